@@ -30,10 +30,11 @@ NVCC_FLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-ffp
                      "-I" + INCLUDE, "-I" + CSRC]
 
 LIB_SOURCES = ["su_io.cpp", "plan.cu", "launch.cu", "search_cmp_plain.cu", "search_cmp_fast.cu",
-               "search_crs_plain.cu", "search_crs_fast.cu", "probe.cu", "noalloc.cu", "neighbours.cu", "de.cu"]
+               "search_crs_plain.cu", "search_crs_fast.cu", "filter.cu", "probe.cu", "noalloc.cu", "neighbours.cu", "de.cu"]
 # the search kernels, compiled a second time with their window checks for the
 # checked library (libsemb_gb300_checked.so, the same ABI)
-SEARCH_SOURCES = ["search_cmp_plain.cu", "search_cmp_fast.cu", "search_crs_plain.cu", "search_crs_fast.cu"]
+SEARCH_SOURCES = ["search_cmp_plain.cu", "search_cmp_fast.cu", "search_crs_plain.cu", "search_crs_fast.cu",
+                  "filter.cu"]
 CHECKED_LIB = os.path.join(OUT, "libsemb_gb300_checked.so")
 
 
@@ -66,7 +67,7 @@ def build(verbose: bool = False) -> str:
     jobs = [(s, ()) for s in LIB_SOURCES] + [(s, ("-DSEMB_CHECKED=1",)) for s in SEARCH_SOURCES] + [
         ("cli.cpp", ("-DSEMB_CLI_METHOD=0",)), ("cli.cpp", ("-DSEMB_CLI_METHOD=1",))]
     # the heaviest translation units (the search kernels) first
-    order = sorted(range(len(jobs)), key=lambda i: not jobs[i][0].startswith("search_"))
+    order = sorted(range(len(jobs)), key=lambda i: not jobs[i][0].startswith(("search_", "filter")))
     with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 4)) as ex:
         done = dict(zip(order, ex.map(lambda i: _compile(*jobs[i]), order)))
     objs = [done[i] for i in range(len(jobs))]

@@ -35,7 +35,8 @@ constexpr int kStages = 3;     // quad stages
 constexpr int kMetaRing = 4;   // chunk metadata and copy descriptors
 constexpr int kRawBufs = 2;    // raw (TMA) buffers
 
-enum : int { CH_PASS_FIRST = 1, CH_PASS_LAST = 2, CH_TASK_LAST = 4, CH_END = 8 };
+// CH_DEAD: the pass has no valid item (semb_filter_kernel)
+enum : int { CH_PASS_FIRST = 1, CH_PASS_LAST = 2, CH_TASK_LAST = 4, CH_END = 8, CH_DEAD = 16 };
 
 // Chunk tags written by the planner next to the chunk metadata.
 struct ChunkTag {
@@ -61,6 +62,7 @@ struct Producer {
   int64_t zpos;     // Z0: the next central trace to add to the pass's sums
   int pseq;         // Z0: passes started; the pass slot is pseq % kZ0Slots
   int zslot, ic_lo; // Z0: the current pass's slot and first C index
+  int drop;         // semb_filter_kernel: traces of the pass on which no item is in range
 };
 
 // Shared-memory layout (bytes), shared by host and device:
@@ -169,6 +171,167 @@ static __device__ __noinline__ void central_add(const KParams& P, int t0s, int64
   }
 }
 
+// The planner warp: plan the next chunk of the stream (its metadata m, tag tg and copy
+// descriptors src) and start its copies into `raw`, counted on `full`.  Z0: see
+// semb_pipe_kernel; z0_base points to its pass slots.
+template <int METHOD, int Z0>
+__device__ __forceinline__ void produce_chunk(const KParams& P, Producer* prod, ChunkMeta* m, ChunkTag* tg, int4* src,
+                                              unsigned char* raw, uint64_t* full, float* z0_base) {
+  const int lane = threadIdx.x & 31;
+  const int c = prod->next;
+  if (prod->task < 0) {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(P.counter, 1);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    __syncwarp();
+    if (t >= (P.ntasks_dev ? *P.ntasks_dev : P.ntasks)) {
+      if (lane == 0) {
+        m->n = 0;
+        m->n_in = 0;
+        m->consumed = 0;
+        m->bytes = 0;
+        tg->flags = CH_END;
+        prod->done = 1;
+        prod->next = c + 1;
+      }
+      __syncwarp();
+      issue_raw(P, m, src, raw, full);
+      return;
+    }
+    const int2 td = P.tasks[t];
+    if (lane == 0) {
+      prod->task = t;
+      prod->cdp = td.x;
+      prod->t0s = td.y;
+      prod->begin = P.ap_off[td.x];
+      prod->end = P.ap_off[td.x + 1];
+      prod->pos = prod->begin;
+      prod->pass = 0;
+      prod->T_lo = P.dt * (float)td.y;
+      prod->T_hi = P.dt * (float)min(td.y + kTB - 1, P.ns - 1);
+      prod->zb = prod->ze = 0;
+      if (Z0) {
+        const int2 zr = P.z0r[td.x];
+        prod->zb = prod->begin + zr.x;
+        prod->ze = prod->zb + zr.y;
+      }
+    }
+    __syncwarp();
+  }
+  const int64_t pos = prod->pos, begin = prod->begin, end = prod->end;
+  const int pass = prod->pass;
+  int flags = pos == begin ? CH_PASS_FIRST : 0;
+  plan_chunk<METHOD, FORM_FAST>(P, P.pass_bounds + pass * 8, pos, end, prod->T_lo, prod->T_hi, m, src, prod->zb,
+                                prod->ze);
+  const int64_t npos = pos + m->consumed;
+  if (Z0) {
+    // the central traces' sums of the pass: a new pass takes the next slot, zeroed;
+    // each chunk adds the next Z0 traces, the pass's last chunk all the rest
+    const int2 pc = P.pass_c[pass];
+    const int slot = pos == begin ? prod->pseq % kZ0Slots : prod->zslot;
+    float* zs = z0_base + (size_t)slot * kZ0SlotFloats;
+    int64_t kb = prod->zpos;
+    if (pos == begin) {
+      kb = prod->zb;
+      for (int q = lane; q < (int)kZ0SlotFloats; q += 32) zs[q] = 0.f;
+    }
+    const int64_t ke = npos >= end ? prod->ze : min(prod->ze, kb + (int64_t)Z0);
+    __syncwarp();
+    central_add(P, prod->t0s, prod->zb, kb, ke, pc.x, pc.y, zs);
+    __syncwarp();
+    if (lane == 0) {
+      if (pos == begin) prod->pseq += 1;
+      prod->zslot = slot;
+      prod->ic_lo = pc.x;
+      prod->zpos = ke;
+      tg->zslot = slot;
+      tg->ic_lo = pc.x;
+    }
+  }
+  if (lane == 0) {
+    if (npos >= end) {
+      flags |= CH_PASS_LAST;
+      prod->pos = begin;
+      prod->pass = pass + 1;
+      if (pass + 1 == P.npass) {
+        flags |= CH_TASK_LAST;
+        prod->task = -1;
+      }
+    } else {
+      prod->pos = npos;
+    }
+    tg->flags = flags;
+    tg->cdp = prod->cdp;
+    tg->t0s = prod->t0s;
+    tg->pass = pass;
+    tg->napert = (int)(end - begin);
+    prod->next = c + 1;
+  }
+  __syncwarp();
+  issue_raw(P, m, src, raw, full);
+}
+
+// One warp has finalized its last pass of a task: the last of the CTA's warps to get
+// here merges every warp's top-4 lists (top_s/top_i/top_k, [kTopK][NT]) into the task's
+// output rows and hands the lists back through merge_done.
+template <int NT>
+__device__ __forceinline__ void merge_task(const KParams& P, const ChunkTag& tg, const float* top_s, const int* top_i,
+                                           const float* top_k, int* merge_cnt, uint64_t* merge_done) {
+  constexpr int K = kTopK;
+  const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  __threadfence_block();
+  __syncwarp();
+  int last = 0;
+  if (lane == 0) last = atomicAdd(merge_cnt, 1) == nwarps - 1;
+  last = __shfl_sync(0xffffffffu, last, 0);
+  if (!last) return;
+  __threadfence_block();
+  float fs[K], fk[K];
+  int fi[K];
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
+    fs[q] = 0.f;
+    fi[q] = 0x7fffffff;
+    fk[q] = 0.f;
+  }
+  for (int w2 = 0; w2 < nwarps; ++w2) {
+    for (int q2 = 0; q2 < K; ++q2) {
+      float cs = top_s[q2 * NT + w2 * 32 + lane];
+      int cidx = top_i[q2 * NT + w2 * 32 + lane];
+      float ck = top_k[q2 * NT + w2 * 32 + lane];
+      if (!(cs > 0.f)) continue;
+#pragma unroll
+      for (int q = 0; q < K; ++q) {
+        if (better(cs, cidx, fs[q], fi[q])) {
+          const float ts = fs[q], tk = fk[q];
+          const int ti = fi[q];
+          fs[q] = cs;
+          fi[q] = cidx;
+          fk[q] = ck;
+          cs = ts;
+          cidx = ti;
+          ck = tk;
+        }
+      }
+    }
+  }
+  const int tt = tg.t0s + lane;
+  if (tt < P.ns) {
+    const int64_t o = (int64_t)tg.cdp * P.ns + tt;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+      P.top_sem[o * kTopK + q] = fs[q];
+      P.top_idx[o * kTopK + q] = fs[q] > 0.f ? fi[q] : -1;
+      P.top_stk[o * kTopK + q] = fk[q];
+    }
+  }
+  __syncwarp();
+  if (lane == 0) {
+    *merge_cnt = 0;
+    mbar_arrive(merge_done);   // the lists may be reused
+  }
+}
+
 // TU: unroll factor of the in-range trace loop (independent work of TU traces in
 // flight per iteration).
 // GLOB: as for semb_search_kernel, the variant may stage less than a whole trace.
@@ -185,7 +348,7 @@ __global__ void __launch_bounds__(NT, MINB) semb_pipe_kernel(KParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const PipeLayout L = pipe_layout(RC, P.cap, P.storage, NT, LAY, Z0 ? 1 : 0);
   float* z0_base = reinterpret_cast<float*>(smem_raw + L.z0);
-  auto z0_slot = [&](int slot) { return z0_base + (size_t)slot * kZ0SlotFloats; };
+  [[maybe_unused]] auto z0_slot = [&](int slot) { return z0_base + (size_t)slot * kZ0SlotFloats; };
   constexpr uint32_t EB = lay_entry_bytes(LAY);   // bytes per staged entry
   uint64_t* raw_full = reinterpret_cast<uint64_t*>(smem_raw);   // [kRawBufs]
   uint64_t* q_full = raw_full + kRawBufs;                        // [kStages]
@@ -245,99 +408,8 @@ __global__ void __launch_bounds__(NT, MINB) semb_pipe_kernel(KParams P) {
   // the planner warp: plan the next chunk of the stream and start its copies
   auto produce = [&]() {
     const int c = prod->next;
-    ChunkMeta* m = meta_at(c);
-    ChunkTag* tg = tag_at(c);
-    int4* src = src_at(c);
-    if (prod->task < 0) {
-      int t = 0;
-      if (lane == 0) t = atomicAdd(P.counter, 1);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      __syncwarp();
-      if (t >= P.ntasks) {
-        if (lane == 0) {
-          m->n = 0;
-          m->n_in = 0;
-          m->consumed = 0;
-          m->bytes = 0;
-          tg->flags = CH_END;
-          prod->done = 1;
-          prod->next = c + 1;
-        }
-        __syncwarp();
-        issue_raw(P, m, src, raw_at(c), &raw_full[c % kRawBufs]);
-        return;
-      }
-      const int2 td = P.tasks[t];
-      if (lane == 0) {
-        prod->task = t;
-        prod->cdp = td.x;
-        prod->t0s = td.y;
-        prod->begin = P.ap_off[td.x];
-        prod->end = P.ap_off[td.x + 1];
-        prod->pos = prod->begin;
-        prod->pass = 0;
-        prod->T_lo = P.dt * (float)td.y;
-        prod->T_hi = P.dt * (float)min(td.y + kTB - 1, P.ns - 1);
-        prod->zb = prod->ze = 0;
-        if (Z0) {
-          const int2 zr = P.z0r[td.x];
-          prod->zb = prod->begin + zr.x;
-          prod->ze = prod->zb + zr.y;
-        }
-      }
-      __syncwarp();
-    }
-    const int64_t pos = prod->pos, begin = prod->begin, end = prod->end;
-    const int pass = prod->pass;
-    int flags = pos == begin ? CH_PASS_FIRST : 0;
-    plan_chunk<METHOD, FORM_FAST>(P, P.pass_bounds + pass * 8, pos, end, prod->T_lo, prod->T_hi, m, src, prod->zb,
-                                  prod->ze);
-    const int64_t npos = pos + m->consumed;
-    if (Z0) {
-      // the central traces' sums of the pass: a new pass takes the next slot, zeroed;
-      // each chunk adds the next Z0 traces, the pass's last chunk all the rest
-      const int2 pc = P.pass_c[pass];
-      const int slot = pos == begin ? prod->pseq % kZ0Slots : prod->zslot;
-      float* zs = z0_slot(slot);
-      int64_t kb = prod->zpos;
-      if (pos == begin) {
-        kb = prod->zb;
-        for (int q = lane; q < (int)kZ0SlotFloats; q += 32) zs[q] = 0.f;
-      }
-      const int64_t ke = npos >= end ? prod->ze : min(prod->ze, kb + (int64_t)Z0);
-      __syncwarp();
-      central_add(P, prod->t0s, prod->zb, kb, ke, pc.x, pc.y, zs);
-      __syncwarp();
-      if (lane == 0) {
-        if (pos == begin) prod->pseq += 1;
-        prod->zslot = slot;
-        prod->ic_lo = pc.x;
-        prod->zpos = ke;
-        tg->zslot = slot;
-        tg->ic_lo = pc.x;
-      }
-    }
-    if (lane == 0) {
-      if (npos >= end) {
-        flags |= CH_PASS_LAST;
-        prod->pos = begin;
-        prod->pass = pass + 1;
-        if (pass + 1 == P.npass) {
-          flags |= CH_TASK_LAST;
-          prod->task = -1;
-        }
-      } else {
-        prod->pos = npos;
-      }
-      tg->flags = flags;
-      tg->cdp = prod->cdp;
-      tg->t0s = prod->t0s;
-      tg->pass = pass;
-      tg->napert = (int)(end - begin);
-      prod->next = c + 1;
-    }
-    __syncwarp();
-    issue_raw(P, m, src, raw_at(c), &raw_full[c % kRawBufs]);
+    produce_chunk<METHOD, Z0>(P, prod, meta_at(c), tag_at(c), src_at(c), raw_at(c), &raw_full[c % kRawBufs],
+                                     z0_base);
   };
 
   int raw_seen = 0;   // chunks whose raw barrier this thread has seen complete
@@ -625,58 +697,7 @@ __global__ void __launch_bounds__(NT, MINB) semb_pipe_kernel(KParams P) {
     if (!(tg.flags & CH_TASK_LAST)) continue;
 
     // ---- task done for this warp; the last warp to get here merges ----
-    __threadfence_block();
-    __syncwarp();
-    int last = 0;
-    if (lane == 0) last = atomicAdd(merge_cnt, 1) == nwarps - 1;
-    last = __shfl_sync(0xffffffffu, last, 0);
-    if (last) {
-      __threadfence_block();
-      float fs[K], fk[K];
-      int fi[K];
-#pragma unroll
-      for (int q = 0; q < K; ++q) {
-        fs[q] = 0.f;
-        fi[q] = 0x7fffffff;
-        fk[q] = 0.f;
-      }
-      for (int w2 = 0; w2 < nwarps; ++w2) {
-        for (int q2 = 0; q2 < K; ++q2) {
-          float cs = top_s[q2 * NT + w2 * 32 + lane];
-          int cidx = top_i[q2 * NT + w2 * 32 + lane];
-          float ck = top_k[q2 * NT + w2 * 32 + lane];
-          if (!(cs > 0.f)) continue;
-#pragma unroll
-          for (int q = 0; q < K; ++q) {
-            if (better(cs, cidx, fs[q], fi[q])) {
-              const float ts = fs[q], tk = fk[q];
-              const int ti = fi[q];
-              fs[q] = cs;
-              fi[q] = cidx;
-              fk[q] = ck;
-              cs = ts;
-              cidx = ti;
-              ck = tk;
-            }
-          }
-        }
-      }
-      const int tt = tg.t0s + lane;
-      if (tt < P.ns) {
-        const int64_t o = (int64_t)tg.cdp * P.ns + tt;
-#pragma unroll
-        for (int q = 0; q < K; ++q) {
-          P.top_sem[o * kTopK + q] = fs[q];
-          P.top_idx[o * kTopK + q] = fs[q] > 0.f ? fi[q] : -1;
-          P.top_stk[o * kTopK + q] = fk[q];
-        }
-      }
-      __syncwarp();
-      if (lane == 0) {
-        *merge_cnt = 0;
-        mbar_arrive(merge_done);   // the lists may be reused
-      }
-    }
+    merge_task<NT>(P, tg, top_s, top_i, top_k, merge_cnt, merge_done);
     ++ntask;
   }
 }

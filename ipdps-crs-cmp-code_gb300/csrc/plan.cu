@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "common.h"
+#include "refine_kernel.cuh"
 #include "pipe_kernel.cuh"
 #include "plan_kernels.cuh"
 #include "semb_kernels.cuh"
@@ -49,12 +50,28 @@ constexpr int kMinStage = 512;
 int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, float c, float* out, cudaStream_t st);
 int launch_repick(int w, const RepickParams& R, cudaStream_t st);
 int launch_crs_de(int w, const DeParams& R, cudaStream_t st);
+bool filter_exists(int form, int w, int brun, int pipe, int lay);
+size_t filter_smem(int form, int storage, int cap);
+int filter_prepare(int form, int w, int storage, size_t smem);
+int launch_filter(int form, int w, int storage, const FilterParams& F, int nwarps, int grid, size_t smem,
+                  cudaStream_t st);
+int launch_refine(int form, int w, int lay, const RefineParams& R, cudaStream_t st);
 
 }  // namespace semb
 
 using namespace semb;
 
 namespace {
+
+// The filter in front of a direct CRS configuration (filter_kernel.cuh): its candidate
+// runs, passes, staging capacity and launch shape.
+struct FilterCfg {
+  int nwarps = 0, npass = 0, cap = 0, nbp = 0, z0 = 0, lay = 0;
+  size_t smem = 0;
+  float dB = 0.f, hbr = 0.f, bmax = 0.f;
+  float4* d_cand = nullptr;
+  float* d_pass_bounds = nullptr;
+};
 
 // One search-kernel configuration: a variant with its candidate table, per-pass
 // parameter bounds, staging capacity, shared memory and residency.
@@ -64,6 +81,7 @@ struct KernelCfg {
   float4* d_cand = nullptr;
   float* d_pass_bounds = nullptr;
   int2* d_pass_c = nullptr;   // Z0 variants: per pass its first C index and C-index count
+  FilterCfg* filter = nullptr;   // owned; null: every candidate is evaluated directly
 };
 
 // A contiguous range of the aperture-sorted work queue, searched by one launch
@@ -126,6 +144,14 @@ struct semb_plan {
   float* d_top_sem = nullptr;
   int32_t* d_top_idx = nullptr;
   float* d_top_stk = nullptr;
+  // CRS filter: the kept runs (per (CDP, t0) their place in a pool); overflowed tasks;
+  // {their count, their queue head, the filter's queue head, -, the pool's entries (64
+  // bits)}, zeroed before every filter launch
+  int2* d_head = nullptr;
+  int2* d_pool = nullptr;
+  int pool_cap = 0;
+  int2* d_fb_tasks = nullptr;
+  int* d_fb_count = nullptr;
   int* d_status = nullptr;
   unsigned long long* d_repicked = nullptr;
   // extra attributes (batched form with attrs = 1)
@@ -212,6 +238,12 @@ void free_cfg(KernelCfg& c) {
   dev_free(c.d_cand);
   dev_free(c.d_pass_bounds);
   dev_free(c.d_pass_c);
+  if (c.filter) {
+    dev_free(c.filter->d_cand);
+    dev_free(c.filter->d_pass_bounds);
+    delete c.filter;
+    c.filter = nullptr;
+  }
   c.variant = -1;
 }
 
@@ -270,6 +302,10 @@ void free_data(semb_plan* pl, bool keep_reusable = false) {
   release(pl->d_top_sem);
   release(pl->d_top_idx);
   release(pl->d_top_stk);
+  release(pl->d_head);
+  release(pl->d_pool);
+  release(pl->d_fb_tasks);
+  release(pl->d_fb_count);
   release(pl->d_sem2);
   release(pl->d_idx2);
   release(pl->d_err64);
@@ -369,6 +405,129 @@ void grid_f64(const semb_params& p, std::vector<double>& abc) {
       abc[3 * (size_t)i + 2] = c0 + pc;
     }
   }
+}
+
+// Per-pass parameter bounds (raw units) of candidate slots of cpp each: bp[0..5] = amin
+// amax bmin bmax cmin cmax of the pass of slot k, grid index gi.
+void widen_bounds(const semb_plan* pl, float* bp, bool first, int gi) {
+  const float v[3] = {pl->ga[gi], pl->gb[gi], pl->gc[gi]};
+  for (int d = 0; d < 3; ++d) {
+    bp[2 * d] = first ? v[d] : std::min(bp[2 * d], v[d]);
+    bp[2 * d + 1] = first ? v[d] : std::max(bp[2 * d + 1], v[d]);
+  }
+}
+
+// Candidate (a, b, c) of grid index gi in sample units, as the batched kernels and the
+// filter take it; .w holds the grid index, -1 for a padding slot.
+float4 sample_candidate(const semb_plan* pl, int gi, bool pad) {
+  const double s1 = pl->idt64, s2 = pl->idt64 * pl->idt64;
+  float4 c = make_float4((float)(pl->g64[3 * (size_t)gi] * s1), (float)(pl->g64[3 * (size_t)gi + 1] * s2),
+                         (float)(pl->g64[3 * (size_t)gi + 2] * s2), 0.f);
+  const int32_t gbits = pad ? -1 : gi;
+  std::memcpy(&c.w, &gbits, 4);
+  return c;
+}
+
+// Put the filter in front of the direct configuration c (variant v) where it pays.
+// SEMB_OK with c.filter null: every candidate is evaluated directly.
+int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_direct, KernelCfg& c) {
+  const semb_params& p = pl->p;
+  const int form = p.mode == SEMB_PLAIN_F32 ? FORM_PLAIN : FORM_FAST;
+  if (p.method != SEMB_CRS || p.ngen > 0 || p.nb < 2 || !filter_exists(form, pl->w, brun, pipe, lay)) return SEMB_OK;
+  const int rc = filter_rc(pl->w), cs = (rc - 1) / 2;
+  const int nruns = (p.nb + rc - 1) / rc;
+  const int64_t total = (int64_t)p.na * p.nc * nruns;
+  // Warp instructions per aperture trace of one task (32 t0): the direct kernels evaluate
+  // every candidate (about 21 instructions batched, 56 plain), the filter every run (90
+  // with its crossings), the refine 32 t0.  Below the line the filter does not pay: a
+  // 9 x 13 x 5 grid with w = 5 took 3.34 ms with it and 3.42 without, 7 x 21 x 7 with few
+  // tasks 2.4 and 1.3.
+  const double direct = (form == FORM_PLAIN ? 56.0 : 21.0) * (double)pl->ncand;
+  const double filtered = 90.0 * (double)total + (form == FORM_PLAIN ? 45.0 : 95.0) * 32.0;
+  if (filtered > 0.9 * direct) return SEMB_OK;
+  // each (A, C) group's B values cut into the fewest runs of at most rc, of equal length
+  // give or take one, each run's middle value in slot cs; padding repeats the run's ends
+  std::vector<int> slots;
+  slots.reserve((size_t)total * rc);
+  int widest = 0;
+  for (int g0 = 0; g0 < pl->ncand; g0 += p.nb)
+    for (int k = 0; k < nruns; ++k) {
+      const int b0 = (int)((int64_t)k * p.nb / nruns), n = (int)((int64_t)(k + 1) * p.nb / nruns) - b0;
+      const int mid = (n - 1) / 2;
+      widest = std::max(widest, n - 1 - mid);
+      for (int q = 0; q < rc; ++q) {
+        const int i = q - cs + mid, ic = std::min(std::max(i, 0), n - 1);
+        slots.push_back(i == ic ? pl->order[g0 + b0 + i] : -1 - pl->order[g0 + b0 + ic]);
+      }
+    }
+  const double dB = (p.b1 - p.b0) * (1.0 / (double)p.nb) * (pl->idt64 * pl->idt64);
+  const double hbr = 0.5 * std::fabs(dB) * widest * (1.0 + 1e-6);
+  // the widest trace of the aperture must expand from a quarter of the record on
+  const double tq = 0.25 * pl->ns, h2 = hbr * (double)p.apm * (double)p.apm;
+  if (!(h2 <= std::min(0.49, 0.0048 * tq) * tq)) return SEMB_OK;
+
+  FilterCfg f;
+  // warps in fours (one per scheduler); the most whose padding stays within 4%
+  int64_t best_tot = INT64_MAX;
+  for (int nw = kFilterNT / 32; nw >= 4; nw -= 4) {
+    const int64_t tot = (total + nw - 1) / nw * nw;
+    if (tot < best_tot) {
+      best_tot = tot;
+      f.nwarps = nw;
+    }
+    if (tot * 100 <= total * 104) break;
+  }
+  f.npass = (int)((total + f.nwarps - 1) / f.nwarps);
+  const int store = form == FORM_PLAIN ? SEMB_STORE_F32 : p.storage;
+  int cap = 16384;
+  while (cap > 64 && filter_smem(form, store, cap) > 226 * 1024) cap -= 64;
+  if (cap < (int)pl->pitch + 16) return SEMB_OK;   // a window may span the whole record
+  f.cap = cap;
+  f.smem = filter_smem(form, store, cap);
+  f.dB = (float)dB;
+  f.hbr = (float)hbr;
+  f.bmax = (float)(std::max(std::fabs(p.b0), std::fabs(p.b1)) * (pl->idt64 * pl->idt64));
+  f.z0 = z0;
+  f.lay = lay;
+  f.nbp = form == FORM_PLAIN ? p.nb : (p.nb + rc_direct - 1) / rc_direct * rc_direct;
+
+  const size_t cpp = (size_t)f.nwarps * rc, npad = (size_t)f.npass * cpp;
+  std::vector<float4> cand(npad);
+  std::vector<float> bounds((size_t)f.npass * 8, 0.f);
+  for (size_t k = 0; k < npad; ++k) {
+    const int sv = slots[std::min(k, slots.size() - 1)];
+    const int gi = sv >= 0 ? sv : -1 - sv;
+    cand[k] = sample_candidate(pl, gi, k >= slots.size() || sv < 0);
+    widen_bounds(pl, &bounds[k / cpp * 8], k % cpp == 0, gi);
+  }
+  // the lists and tables; without the memory for them the search is direct
+  const size_t nout = (size_t)pl->ncdps * pl->ns;
+  pl->pool_cap = (int)std::min<size_t>(nout * kFilterPool + 4096, INT32_MAX);
+  if (dev_reuse(pl, &pl->d_head, nout) != SEMB_OK || dev_reuse(pl, &pl->d_pool, (size_t)pl->pool_cap) != SEMB_OK ||
+      dev_reuse(pl, &pl->d_fb_tasks, pl->ntasks) != SEMB_OK || dev_reuse(pl, &pl->d_fb_count, 6) != SEMB_OK ||
+      dev_alloc(&f.d_cand, npad) != SEMB_OK || dev_alloc(&f.d_pass_bounds, bounds.size()) != SEMB_OK) {
+    cudaGetLastError();
+    dev_free(f.d_cand);
+    dev_free(f.d_pass_bounds);
+    return SEMB_OK;
+  }
+  cudaError_t e = cudaMemcpyAsync(f.d_cand, cand.data(), npad * sizeof(float4), cudaMemcpyHostToDevice, pl->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(f.d_pass_bounds, bounds.data(), bounds.size() * 4, cudaMemcpyHostToDevice, pl->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(pl->stream);
+  int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, f.smem) : SEMB_OK;
+  if (e != cudaSuccess || rc_prep != SEMB_OK) {
+    dev_free(f.d_cand);
+    dev_free(f.d_pass_bounds);
+    SEMB_CUDA(e);
+    return rc_prep;
+  }
+  c.filter = new (std::nothrow) FilterCfg(f);
+  if (!c.filter) {
+    dev_free(f.d_cand);
+    dev_free(f.d_pass_bounds);
+  }
+  return SEMB_OK;
 }
 
 // Launch configuration of search-kernel variant v into `out`: candidates per pass
@@ -471,36 +630,20 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   const int npad = npass * cpp;
   std::vector<float4> cand(npad);
   std::vector<float> bounds((size_t)npass * 8, 0.f);
-  const double s1 = pl->idt64, s2 = pl->idt64 * pl->idt64;
   for (int k = 0; k < npad; ++k) {
     // padding slots repeat a real candidate's parameters (so the pass bounds are
     // unchanged) with grid index -1: they are evaluated but never picked
     const int sv = slots[std::min(k, nslots - 1)];
     const bool pad = k >= nslots || sv < 0;
     const int gi = sv >= 0 ? sv : -1 - sv;
-    float4 c;
+    float4 c = sample_candidate(pl, gi, pad);
     if (form == FORM_PLAIN) {
-      c = make_float4(pl->ga[gi], pl->gb[gi], pl->gc[gi], 0.f);
-    } else {
-      c = make_float4((float)(pl->g64[3 * (size_t)gi] * s1), (float)(pl->g64[3 * (size_t)gi + 1] * s2),
-                      (float)(pl->g64[3 * (size_t)gi + 2] * s2), 0.f);
+      c.x = pl->ga[gi];
+      c.y = pl->gb[gi];
+      c.z = pl->gc[gi];
     }
-    int32_t gbits = pad ? -1 : gi;
-    std::memcpy(&c.w, &gbits, 4);
     cand[k] = c;
-    float* bp = &bounds[(size_t)(k / cpp) * 8];
-    if (k % cpp == 0) {
-      bp[0] = bp[1] = pl->ga[gi];
-      bp[2] = bp[3] = pl->gb[gi];
-      bp[4] = bp[5] = pl->gc[gi];
-    } else {
-      bp[0] = std::min(bp[0], pl->ga[gi]);
-      bp[1] = std::max(bp[1], pl->ga[gi]);
-      bp[2] = std::min(bp[2], pl->gb[gi]);
-      bp[3] = std::max(bp[3], pl->gb[gi]);
-      bp[4] = std::min(bp[4], pl->gc[gi]);
-      bp[5] = std::max(bp[5], pl->gc[gi]);
-    }
+    widen_bounds(pl, &bounds[(size_t)(k / cpp) * 8], k % cpp == 0, gi);
   }
   KernelCfg c;
   if (dev_alloc(&c.d_cand, npad) != SEMB_OK || dev_alloc(&c.d_pass_bounds, bounds.size()) != SEMB_OK ||
@@ -527,6 +670,11 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   c.cap = cap;
   c.smem = smem;
   c.occ = occ;
+  const int frc = attach_filter(pl, brun, pipe, lay, z0, rc, c);
+  if (frc != SEMB_OK) {
+    free_cfg(c);
+    return frc;
+  }
   free_cfg(out);
   out = c;
   drop_graph(pl);
@@ -1114,6 +1262,58 @@ KParams make_kparams_cfg(semb_plan* pl, const KernelCfg& cfg, const int2* tasks,
   return P;
 }
 
+// The search of tasks[0, ntasks) with configuration cfg on stream st, work-queue head
+// `counter` (zeroed by the caller; the plain form has none): the direct kernel, or the filter, the refine of what it kept and
+// the direct kernel on the tasks whose lists overflowed.  grid: the direct kernel's.
+int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int ntasks, int grid, int* counter,
+                   cudaStream_t st, int* launches) {
+  const semb_params& p = pl->p;
+  const int form = p.mode == SEMB_PLAIN_F32 ? FORM_PLAIN : FORM_FAST;
+  KParams P = make_kparams_cfg(pl, cfg, tasks, ntasks, counter);
+  if (const FilterCfg* f = cfg.filter) {
+    SEMB_CUDA(cudaMemsetAsync(pl->d_fb_count, 0, 6 * sizeof(int), st));
+    FilterParams F{};
+    F.k = P;
+    F.k.cand = f->d_cand;
+    F.k.pass_bounds = f->d_pass_bounds;
+    F.k.npass = f->npass;
+    F.k.cpp = f->nwarps * filter_rc(pl->w);
+    F.k.cap = f->cap;
+    F.k.dB = f->dB;
+    F.k.hbr = f->hbr;
+    F.k.bmax = f->bmax;
+    F.k.counter = pl->d_fb_count + 2;
+    F.head = pl->d_head;
+    F.pool = pl->d_pool;
+    F.pool_cap = pl->pool_cap;
+    F.pool_count = reinterpret_cast<unsigned long long*>(pl->d_fb_count + 4);
+    F.fb_tasks = pl->d_fb_tasks;
+    F.fb_count = pl->d_fb_count;
+    F.kappa = form == FORM_PLAIN ? 16.f : 8.f;
+    SEMB_TRY(launch_filter(form, pl->w, P.storage, F, f->nwarps, std::min(ntasks, pl->sms), f->smem, st));
+    RefineParams R{};
+    R.k = P;
+    R.head = pl->d_head;
+    R.pool = pl->d_pool;
+    R.runs = f->d_cand;
+    R.tasks = tasks;
+    R.ntasks = ntasks;
+    R.na = p.na;
+    R.nb = p.nb;
+    R.nc = p.nc;
+    R.nbp = f->nbp;
+    R.z0 = f->z0;
+    SEMB_TRY(launch_refine(form, pl->w, f->lay, R, st));
+    P.tasks = pl->d_fb_tasks;
+    P.ntasks_dev = pl->d_fb_count;
+    P.counter = pl->d_fb_count + 1;
+    if (launches) *launches += 2;
+  }
+  SEMB_TRY(launch_search(p.method, form, pl->w, cfg.variant, P, cfg.nwarps, grid, cfg.smem, st));
+  if (launches) ++*launches;
+  return SEMB_OK;
+}
+
 KParams make_kparams(semb_plan* pl, int bucket) {
   const Bucket& b = pl->buckets[bucket];
   return make_kparams_cfg(pl, b.cfg, pl->d_tasks + b.begin, b.end - b.begin, pl->d_counter + bucket);
@@ -1193,10 +1393,8 @@ int enqueue_run(semb_plan* pl, bool timed) {
     Bucket run = pl->buckets[i];
     run.end = pl->buckets[j - 1].end;
     if (run.end > run.begin) {
-      const KParams Pb = make_kparams_cfg(pl, run.cfg, pl->d_tasks + run.begin, run.end - run.begin, pl->d_counter + i);
-      SEMB_TRY(launch_search(p.method, form, pl->w, run.cfg.variant, Pb, run.cfg.nwarps, bucket_grid(pl, run),
-                             run.cfg.smem, st));
-      ++launches;
+      SEMB_TRY(enqueue_search(pl, run.cfg, pl->d_tasks + run.begin, run.end - run.begin, bucket_grid(pl, run),
+                              pl->d_counter + i, st, &launches));
     }
     i = j;
   }
@@ -1267,16 +1465,13 @@ int enqueue_streamed(semb_plan* pl, const semb_gather_view* g) {
   SEMB_CUDA(cudaMemsetAsync(pl->d_chunk_counter, 0, nk * sizeof(int), st));
   SEMB_CUDA(cudaEventRecord(pl->ev[0], st));
   const Bucket& b = pl->buckets[0];
-  const int form = FORM_FAST;
   int launches = 0;
   for (int k = 0; k < nk; ++k) {
     const int n = pl->chunk_task[k + 1] - pl->chunk_task[k];
     if (n == 0) continue;
     SEMB_CUDA(cudaStreamWaitEvent(st, pl->chunk_done[pl->chunk_need[k]], 0));
-    const KParams P = make_kparams_cfg(pl, b.cfg, pl->d_tasks + pl->chunk_task[k], n, pl->d_chunk_counter + k);
-    SEMB_TRY(launch_search(p.method, form, pl->w, b.cfg.variant, P, b.cfg.nwarps, std::min(n, pl->sms * b.cfg.occ),
-                           b.cfg.smem, st));
-    ++launches;
+    SEMB_TRY(enqueue_search(pl, b.cfg, pl->d_tasks + pl->chunk_task[k], n, std::min(n, pl->sms * b.cfg.occ),
+                            pl->d_chunk_counter + k, st, &launches));
   }
   SEMB_CUDA(cudaStreamWaitEvent(st, pl->chunk_done[nk - 1], 0));
   if (p.method == SEMB_CRS) {
@@ -1315,7 +1510,7 @@ int count_chunk_launches(const semb_plan* pl, const semb_plan::RunChunk& ch, int
   for (int i = 0; i < nb;) {
     int j = i + 1;
     while (j < nb && pl->buckets[j].cfg.variant == pl->buckets[i].cfg.variant) ++j;
-    if (ch.bucket_begin[j] > ch.bucket_begin[i]) ++*n;
+    if (ch.bucket_begin[j] > ch.bucket_begin[i]) *n += pl->buckets[i].cfg.filter ? 3 : 1;
     i = j;
   }
   return SEMB_OK;
@@ -1387,10 +1582,8 @@ int enqueue_chunk(semb_plan* pl, const semb_plan::RunChunk& ch, int* launches) {
     const int t0 = ch.bucket_begin[i], n = ch.bucket_begin[j] - t0;
     if (n > 0) {
       const KernelCfg& cfg = pl->buckets[i].cfg;
-      const KParams P = make_kparams_cfg(pl, cfg, pl->d_chunk_tasks + t0, n, pl->d_counter + i);
-      SEMB_TRY(launch_search(p.method, FORM_FAST, pl->w, cfg.variant, P, cfg.nwarps, std::min(n, pl->sms * cfg.occ),
-                             cfg.smem, st));
-      ++*launches;
+      SEMB_TRY(enqueue_search(pl, cfg, pl->d_chunk_tasks + t0, n, std::min(n, pl->sms * cfg.occ), pl->d_counter + i,
+                              st, launches));
     }
     i = j;
   }
@@ -1656,13 +1849,12 @@ int semb_plan_autotune(semb_plan* pl, int32_t* chosen, double* ms_of_variant) {
         fits[v] = 0;
         continue;
       }
-      const KParams P = make_kparams_cfg(pl, guard.trial, d_sample, S, pl->d_counter);
       const int grid = form == FORM_PLAIN ? S : std::min(S, pl->sms * guard.trial.occ);
       float ms = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
         SEMB_CUDA(cudaMemsetAsync(pl->d_counter, 0, sizeof(int), st));
         SEMB_CUDA(cudaEventRecord(pl->ev[4], st));
-        SEMB_TRY(launch_search(p.method, form, pl->w, v, P, guard.trial.nwarps, grid, guard.trial.smem, st));
+        SEMB_TRY(enqueue_search(pl, guard.trial, d_sample, S, grid, pl->d_counter, st, nullptr));
         SEMB_CUDA(cudaEventRecord(pl->ev[5], st));
         SEMB_CUDA(cudaStreamSynchronize(st));
         float t = 0.f;

@@ -106,6 +106,7 @@ struct KParams {
   // tasks (cdp, t0_start)
   const int2* tasks;
   int ntasks;
+  const int* ntasks_dev;        // not null: the task count, in device memory
   int* counter;                 // work-queue head (fast form)
   // sampling
   int ns;
@@ -129,6 +130,11 @@ struct KParams {
   const float* cvals;
   const int2* pass_c;
   int nc_grid;
+  // semb_filter_kernel: the B step of the grid, half the widest run's B range and the
+  // largest |B|, in sample units (samples^2 per m^2)
+  float dB;
+  float hbr;
+  float bmax;
 };
 
 // Z0 variants: the most C indices one pass may span, and the pass slots of the central
@@ -335,7 +341,7 @@ __host__ __device__ inline SmemLayout smem_layout(int form, int rc, int cap, int
 // exact, because an out-of-range trace only counts in err = N_ap - M.
 template <int METHOD>
 __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_lo, float T_hi, float idt,
-                                             int tau, int ns, int& lo, int& hi, bool& inrange) {
+                                             int tau, int ns, int& lo, int& hi, bool& inrange, float& smin) {
   inrange = false;
   float t2min, t2max;
   if (METHOD == METHOD_CMP) {
@@ -362,7 +368,7 @@ __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_
     hi = ns - 1;
     return true;
   }
-  float smin = t2min > 0.f ? sqrtf(t2min) * idt : 0.f;
+  smin = t2min > 0.f ? sqrtf(t2min) * idt : 0.f;
   float smax = sqrtf(t2max) * idt;
   smin = fminf(smin, (float)ns + 8.f);
   smax = fminf(smax, (float)ns + 8.f);
@@ -378,16 +384,28 @@ __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_
   return lo <= hi;
 }
 
+// semb_filter_kernel: half the spread of a B run's traveltimes about its centre is at
+// most `h2` / t samples (h2 = dm^2 times half the run's B range), t >= smin.  The run
+// expands about its centre when that stays below half a sample, so that at most one
+// sample boundary lies between any item and the centre, and when the expansion's
+// first dropped term, h^3 / (2 t^2) samples for a half spread h, is below the rounding
+// of an FP32 traveltime (t 2^-24): h <= 0.0048 t.
+__device__ __forceinline__ bool moment_narrow(float h2, float smin) {
+  return h2 <= fminf(0.49f, 0.0048f * smin) * smin;
+}
+
 // Warp 0: choose the entries of the next chunk starting at ap_pos and record, per
 // entry, its geometry, its buffer offset (minus the window start, so that an item
 // indexes with it - tau directly) and its source window (trace, first sample,
 // length, offset) in `src`.  Aperture traces on which no item can be in range are
 // consumed without an entry.  meta->n counts entries, meta->consumed the aperture
 // traces the chunk covers.  Fast form: entries on which every item is in range go
-// to the front slots, the others to the back (entry_slot).  Windows are aligned to ALIGN samples: 4 for FP32 bulk
+// to the front slots, the others to the back (entry_slot); MOM keeps only entries
+// whose B runs expand about their centre (moment_narrow) in front, and raw[] says which of
+// the others do.  Windows are aligned to ALIGN samples: 4 for FP32 bulk
 // copies (16 bytes), 8 for the fast form's raw windows.  Buffer units: floats
 // (plain) or one 16-byte entry per sample (fast).
-template <int METHOD, int FORM>
+template <int METHOD, int FORM, bool MOM = false>
 __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, int64_t ap_end, float T_lo,
                            float T_hi, ChunkMeta* meta, int4* src, int64_t skip_b = 0, int64_t skip_e = 0) {
   const int lane = threadIdx.x & 31;
@@ -406,9 +424,15 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
     int tr = 0;
     float sc = 1.0f;
     bool glob = false;
+    [[maybe_unused]] bool narrow = false;
     if (have) {
       g = P.ap_geo[k];
-      keep = trace_window<METHOD>(pb, g, T_lo, T_hi, P.idt, P.tau, P.ns, lo, hi, inr);
+      float smin = 0.f;
+      keep = trace_window<METHOD>(pb, g, T_lo, T_hi, P.idt, P.tau, P.ns, lo, hi, inr, smin);
+      if constexpr (MOM) {
+        narrow = moment_narrow(P.hbr * fabsf(g.y), smin);
+        inr = inr && narrow;
+      }
       // a trace of the central CDP at zero midpoint distance whose sums the pass shares
       // over A and B (Z0 variants) is left out
       if (k >= skip_b && k < skip_e && g.x == 0.f) keep = false;
@@ -449,7 +473,8 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
       g.w = __int_as_float(glob ? kGlobalEntry : off - lo);
       meta->geo[e] = g;
       meta->scale[e] = sc;
-      meta->raw[e] = glob ? tr : off + 8 * rank;
+      if constexpr (MOM) meta->raw[e] = narrow ? 1 : 0;
+      else meta->raw[e] = glob ? tr : off + 8 * rank;
       src[e] = make_int4(tr, lo, len, off);   // len 0: nothing to copy or convert
     }
     const int nhave = __popc(__ballot_sync(0xffffffffu, have));
@@ -1120,6 +1145,7 @@ template <int METHOD, int FORM, int W, int RC, int MINB, int LAY, bool BRUN, int
           bool XP = false>
 __global__ void __launch_bounds__(NT, MINB) semb_search_kernel(KParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  if (FORM == FORM_PLAIN && P.ntasks_dev && (int)blockIdx.x >= *P.ntasks_dev) return;
   const SmemLayout L = smem_layout(FORM, RC, P.cap, P.storage, NT, LAY);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw);   // [2]
   int* ctl = reinterpret_cast<int*>(smem_raw + 16);
