@@ -26,7 +26,7 @@
 //                E = sum_j v_j^2, G = sum_j v_j d_j, H = sum_j d_j^2
 //
 // (the r^4 term, k2^2 H, is below 4e-7 of E at the widest run the planner admits).  One
-// trace costs a lane about 46 instructions for the whole run, where the direct kernels
+// trace costs a lane about 40 instructions for the whole run, where the direct kernels
 // spend about 20 on every item.
 //
 // Crossings.  Where some item of the run lies across a sample boundary from the centre,
@@ -56,21 +56,28 @@
 // per chunk.  The pipeline otherwise follows semb_pipe_kernel: a rotating planner warp,
 // mbarrier hand-offs, a work queue, the last warp of a task merging its lists.
 //
-// What bounds it: instruction issue (about 46 per trace and run, 20 to 40 for the
-// crossings, the rest staging and planning), issued on about 70% of cycles.  Measured on
-// GB300, whole search without the FP64 re-pick, direct kernel -> filter and refine: 64 CDPs
-// of the 500 x 48 CRS line (21 x 21 x 21, FP16) 162 -> 73 ms; 128 CDPs with apertures of
-// 50 to 2000 traces 386 -> 172 ms; 48 such CDPs with 31 x 31 x 31 candidates (BF16)
-// 961 -> 382 ms; plain form, 12 CDPs of the line 99 -> 12 ms.
+// What bounds it: instruction issue.  On 16 CDPs of the 500 x 48 line with runs of 21 the
+// main loop (about 40 instructions per trace and run) issues on every cycle and takes 30%
+// of the time, the crossings (about 100 per noted trace of the busiest lane, on 56% of
+// cycles) 30%, the traces at the record's ends 10 to 15%, and the rest is the planner's and
+// the copies' latency, hidden only in part.  Long runs pay: 21 B values as one run of 22
+// slots at 384 threads took 29.5 ms where two runs of 12 slots at 512 threads took 36.2 (32
+// CDPs of the line), 31 as one of 32 slots at 256 threads 130 against 147 as two of 16.  The
+// second-order terms only where they count (moment_linear) gave 2%, the crossings above
+// and below the centre apart (half the slots each) 7%; two noted traces at a time was 10%
+// slower, and so was the main loop unrolled by four.
+// Measured on GB300, whole pass with the FP64 re-pick, direct kernels -> filter and refine:
+// 64 CDPs of the line (21 x 21 x 21, FP16) 172.3 -> 61.7 ms; 128 CDPs with apertures of 50
+// to 2000 traces 832 -> 281 ms; 48 such CDPs with 31 x 31 x 31 candidates (BF16) 621 -> 172
+// ms; plain form, 12 CDPs of the line 99.6 -> 9.3 ms.
 #pragma once
+
+#include <type_traits>
 
 #include "pipe_kernel.cuh"
 
 namespace semb {
 
-// slots per run: the per-item sums (w + 1 per slot) fill the register budget
-__host__ __device__ constexpr int filter_rc(int w) { return w == 5 ? 8 : 12; }
-constexpr int kFilterNT = 512;     // threads per CTA, one CTA per SM
 constexpr int kFilterList = 6;     // runs kept per thread
 constexpr int kFilterPool = 6;     // output pool: kept runs per (CDP, t0) on average
 
@@ -82,7 +89,7 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
 }
 
 struct FilterParams {
-  KParams k;               // geometry, queue, candidate runs ([npass * warps][filter_rc(w)]), staging
+  KParams k;               // geometry, queue, candidate runs ([npass * warps][RC]), staging
   int2* head;              // [ncdps][ns]: (first entry, entries) in the pool; entries -1: the
                            // task goes to the direct kernel
   int2* pool;              // entries (run, slot mask)
@@ -106,14 +113,14 @@ struct FilterLayout {
   size_t prod, meta, tag, src, list, plane, plane_stride, raw, raw_stride, total;
 };
 
-__host__ __device__ inline FilterLayout filter_layout(int cap, bool f32, int kt) {
+__host__ __device__ inline FilterLayout filter_layout(int cap, bool f32, int kt, int nt) {
   FilterLayout L;
   L.prod = 128;
   L.meta = L.prod + align128(sizeof(Producer));
   L.tag = L.meta + kMetaRing * kMetaBytes;
   L.src = L.tag + align128(kMetaRing * sizeof(ChunkTag));
   L.list = L.src + (size_t)kMetaRing * kMaxChunk * 16;
-  L.plane = L.list + (size_t)(3 * kFilterList + kt + 1) * kFilterNT * 4;
+  L.plane = L.list + (size_t)(3 * kFilterList + kt + 1) * nt * 4;
   L.plane_stride = align128(((size_t)cap + kZeroSlots) * 4);
   L.raw = L.plane + kStages * L.plane_stride;
   L.raw_stride = f32 ? 0 : align128((size_t)cap * 2);
@@ -142,6 +149,8 @@ struct MomentSums {
   }
   // one trace: window samples at address a, weight x, expansion k1 and k2n = k1^2 / t
   // (k2 = -k2n / 2; the factor is applied at the end of the pass)
+  // QUAD: with the terms of k2n (else they are below the rounding, moment_linear)
+  template <bool QUAD>
   __device__ __forceinline__ void add(uint32_t a, float x, float k1, float k2n) {
     float s[W + 1];
 #pragma unroll
@@ -151,7 +160,7 @@ struct MomentSums {
     const float ws = fmaf(ds, x, s[JS]);
     vs += ws;
     n1s = fmaf(ds, k1, n1s);
-    n2s = fmaf(ds, k2n, n2s);
+    if (QUAD) n2s = fmaf(ds, k2n, n2s);
     float G = ws * ds, H = ds * ds;
     e0.x = fmaf(ws, ws, e0.x);
 #pragma unroll
@@ -161,7 +170,7 @@ struct MomentSums {
       const float2 w = __ffma2_rn(d, xx, lo);
       v[i] = __fadd2_rn(v[i], w);
       n1[i] = __ffma2_rn(d, kk1, n1[i]);
-      n2[i] = __ffma2_rn(d, kk2, n2[i]);
+      if (QUAD) n2[i] = __ffma2_rn(d, kk2, n2[i]);
       e0 = __ffma2_rn(w, w, e0);
       G = fmaf(w.x, d.x, fmaf(w.y, d.y, G));
       H = fmaf(d.x, d.x, fmaf(d.y, d.y, H));
@@ -169,8 +178,10 @@ struct MomentSums {
     e1 = fmaf(k1, G, e1);
     const float aH = k1 * H;
     e2 = fmaf(aH, k1, e2);
-    e2 = fmaf(-k2n, G, e2);
-    e3 = fmaf(k2n, aH, e3);
+    if (QUAD) {
+      e2 = fmaf(-k2n, G, e2);
+      e3 = fmaf(k2n, aH, e3);
+    }
     h += H;
   }
   // num_j at slot offsets rr
@@ -234,16 +245,17 @@ __device__ __forceinline__ void convert_windows(const KParams& P, const ChunkMet
 }
 
 // W: window.  F32: stage the FP32 store (plain form, FP32 batched store).  KT: how many
-// best candidates the search keeps per (CDP, t0).
-template <int W, bool F32, int KT>
-__global__ void __launch_bounds__(kFilterNT, 1) semb_filter_kernel(FilterParams FP) {
-  static_assert(W == 1 || W == 3 || W == 5, "CRS windows");
-  constexpr int RC = filter_rc(W), NT = kFilterNT, KL = kFilterList;
+// best candidates the search keeps per (CDP, t0).  RC: slots per run (even).  NT: threads
+// per CTA, one CTA per SM.
+template <int W, bool F32, int KT, int RC, int NT>
+__global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
+  static_assert((W == 1 || W == 3 || W == 5) && RC % 2 == 0 && RC <= 32, "CRS windows; slot pairs and masks");
+  constexpr int KL = kFilterList;
   constexpr int RP = RC / 2;
   constexpr int CS = (RC - 1) / 2;   // the centre slot
   const KParams& P = FP.k;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const FilterLayout L = filter_layout(P.cap, F32, KT);
+  const FilterLayout L = filter_layout(P.cap, F32, KT, NT);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);   // copies landed: [kStages] (F32) or [kRawBufs]
   uint64_t* q_full = full + kStages;                         // [kStages] (16-bit: converted)
   uint64_t* q_empty = q_full + kStages;                      // [kStages]
@@ -462,119 +474,109 @@ __global__ void __launch_bounds__(kFilterNT, 1) semb_filter_kernel(FilterParams 
     const uint32_t plane = smem_u32(plane_at(c));
     const uint32_t top = plane + 4u * (uint32_t)P.cap;
     const uint32_t base0 = plane - 4u * (0x4B000000u + (uint32_t)P.tau);
-    uint32_t mask[kMaxChunk / 32];   // traces with a crossing
+    // traces whose run crosses the sample boundary above, below the centre
+    uint32_t up_mask[kMaxChunk / 32], dn_mask[kMaxChunk / 32];
+    auto front = [&](auto quad) {
+      constexpr bool QUAD = decltype(quad)::value;
 #pragma unroll
-    for (int b = 0; b < kMaxChunk / 32; ++b) {
-      mask[b] = 0;
-      const int e1 = min(n_in, 32 * b + 32);
+      for (int b = 0; b < kMaxChunk / 32; ++b) {
+        uint32_t um = 0, dm = 0;
+        const int e1 = min(n_in, 32 * b + 32);
 #pragma unroll 2
-      for (int e = 32 * b; e < e1; ++e) {
-        const float4 g = meta->geo[e];
-        const float u = fmaf(ca, g.x, T);
-        const float q = fmaf(cb, g.y, fmaf(u, u, cc * g.z));
-        const float t = sqrt_fast(q), ti = rsqrt_fast(q);
-        const float y = __fadd_rz(t, 8388608.0f);
-        const float x = t - (y - 8388608.0f);
-        const float k1 = (hdB * g.y) * ti;
-        const float k2n = (k1 * k1) * ti;
-        const uint32_t a = min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top);
-        if constexpr (SEMB_CHECKED) {
-          report_window(P.status, __float_as_int(y) - 0x4B000000 - P.tau + __float_as_int(g.w), W, src_at(c)[e], tg.cdp,
-                        t0);
+        for (int e = 32 * b; e < e1; ++e) {
+          const float4 g = meta->geo[e];
+          const float u = fmaf(ca, g.x, T);
+          const float q = fmaf(cb, g.y, fmaf(u, u, cc * g.z));
+          const float t = sqrt_fast(q), ti = rsqrt_fast(q);
+          const float y = __fadd_rz(t, 8388608.0f);
+          const float x = t - (y - 8388608.0f);
+          const float k1 = (hdB * g.y) * ti;
+          const uint32_t a = min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top);
+          if constexpr (SEMB_CHECKED) {
+            report_window(P.status, __float_as_int(y) - 0x4B000000 - P.tau + __float_as_int(g.w), W, src_at(c)[e],
+                          tg.cdp, t0);
+          }
+          ms.template add<QUAD>(a, x, k1, QUAD ? (k1 * k1) * ti : 0.f);
+          const float h = k1 * rmax;
+          if (x + h >= 1.0f) um |= 1u << (e - 32 * b);
+          if (x < h) dm |= 1u << (e - 32 * b);
         }
-        ms.add(a, x, k1, k2n);
-        if (fmaf(fabsf(k1), rmax, fabsf(x - 0.5f)) >= 0.5f) mask[b] |= 1u << (e - 32 * b);
+        up_mask[b] = um;
+        dn_mask[b] = dm;
       }
-    }
-    // crossings: each lane takes its next noted trace until none has one
-    while (__any_sync(0xffffffffu, (mask[0] | mask[1] | mask[2] | mask[3]) != 0)) {
-      const bool have = (mask[0] | mask[1] | mask[2] | mask[3]) != 0;
-      int e = 0;
-      if (mask[0]) {
-        e = __ffs(mask[0]) - 1;
-        mask[0] &= mask[0] - 1;
-      } else if (mask[1]) {
-        e = 31 + __ffs(mask[1]);
-        mask[1] &= mask[1] - 1;
-      } else if (mask[2]) {
-        e = 63 + __ffs(mask[2]);
-        mask[2] &= mask[2] - 1;
-      } else if (mask[3]) {
-        e = 95 + __ffs(mask[3]);
-        mask[3] &= mask[3] - 1;
-      }
-      const float4 g = meta->geo[e];
-      const float u = fmaf(ca, g.x, T);
-      const float q = fmaf(cb, g.y, fmaf(u, u, cc * g.z));
-      const float t = sqrt_fast(q), ti = rsqrt_fast(q);
-      const float y = __fadd_rz(t, 8388608.0f);
-      const float x = t - (y - 8388608.0f);
-      const float k1 = (hdB * g.y) * ti;
-      const float k2 = -0.5f * ((k1 * k1) * ti);
-      const bool hi = x >= 0.5f;
-      // the boundary samples p_1 .. p_W with their neighbours p_0, p_W+1: the window
-      // itself for a crossing upwards, one sample earlier for one downwards
-      const uint32_t a = min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top) - (hi ? 0u : 4u);
-      if constexpr (SEMB_CHECKED) {
-        if (have)
-          report_window(P.status, __float_as_int(y) - 0x4B000000 - P.tau + __float_as_int(g.w) - (hi ? 0 : 1), W + 1,
-                        src_at(c)[e], tg.cdp, t0);
-      }
-      float p[W + 2];
-#pragma unroll
-      for (int j = 0; j < W + 2; ++j) p[j] = lds32(a + 4u * j);
-      // distance beyond the boundary z_r = z0 + sz (k1 r + k2 r^2); beyond it sample j is
-      // p_j+1 + e_j z + c_j z with e_j the centre interval's slope along z
-      const float z0 = hi ? x - 1.0f : -x;
-      const float sz = hi ? 1.0f : -1.0f;
-      float cj[W], q1 = 0.f, q2 = 0.f;
-#pragma unroll
-      for (int j = 0; j < W; ++j) {
-        const float dm = p[j + 1] - p[j], dp = p[j + 2] - p[j + 1];
-        cj[j] = have ? dp - dm : 0.f;
-        const float ej = hi ? dm : -dp;
-        q1 = fmaf(2.f * cj[j], p[j + 1], q1);
-        q2 = fmaf(cj[j], fmaf(2.f, ej, cj[j]), q2);
-      }
-      const float2 z02 = make_float2(z0, z0), a1 = make_float2(sz * k1, sz * k1), a2 = make_float2(sz * k2, sz * k2);
-      const float2 q12 = make_float2(q1, q1), q22 = make_float2(q2, q2);
-#pragma unroll
-      for (int pr = 0; pr < RP; ++pr) {
-        const float2 rr = make_float2((float)(2 * pr - CS), (float)(2 * pr + 1 - CS));
-        float2 z = __ffma2_rn(rr, __ffma2_rn(rr, a2, a1), z02);
-        z = make_float2(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f));
-#pragma unroll
-        for (int j = 0; j < W; ++j) inum[j][pr] = __ffma2_rn(make_float2(cj[j], cj[j]), z, inum[j][pr]);
-        iden[pr] = __ffma2_rn(z, __ffma2_rn(z, q22, q12), iden[pr]);
-      }
-    }
-    // the other traces.  A narrow one whose run is well inside the record on this lane
-    // joins the moments; one whose run is well outside is a miss for every item; where the
-    // run straddles an end, and for wide traces, each item goes on its own with range
-    // checks: an out-of-range item reads the zero block with weight 0 and does not count
+    };
+    const bool quad = meta->quad != 0;
+    if (quad) front(std::true_type{});
+    else front(std::false_type{});
+    // the other traces.  Wide ones in the record: every item on its own.  A narrow one whose
+    // run is well inside the record on this lane joins the moments (and the crossings); one
+    // whose run is well outside is a miss for every item; where the run straddles an end,
+    // and for the other wide traces, each item goes on its own with range checks: an
+    // out-of-range item reads the zero block with weight 0 and does not count
     for (int e = kMaxChunk - (n - n_in); e < kMaxChunk; ++e) {
       const float4 g = meta->geo[e];
       const int soff = __float_as_int(g.w);
       const float u = fmaf(ca, g.x, T);
       const float q0 = fmaf(u, u, cc * g.z);
+      const int kind = meta->raw[e];
+      if (kind == 2) {
+        // wide, every item in range: items two at a time, no range checks
+        const float qc = fmaf(cb, g.y, q0), qs = P.dB * g.y;
+        const uint32_t base = base0 + 4u * (uint32_t)soff;
+#pragma unroll
+        for (int pr = 0; pr < RP; ++pr) {
+          const float2 rr = make_float2((float)(2 * pr - CS), (float)(2 * pr + 1 - CS));
+          const float2 q = __ffma2_rn(rr, make_float2(qs, qs), make_float2(qc, qc));
+          const float2 t = make_float2(sqrt_fast(q.x), sqrt_fast(q.y));
+          const float2 y = __fadd2_rz(t, make_float2(8388608.0f, 8388608.0f));
+          const float2 x = __ffma2_rn(__fadd2_rn(y, make_float2(-8388608.0f, -8388608.0f)), make_float2(-1.f, -1.f), t);
+          // a padding slot's window may not be staged: the address stays in the plane
+          const uint32_t ax = max(min(__float_as_uint(y.x) * 4u + base, top), plane);
+          const uint32_t ay = max(min(__float_as_uint(y.y) * 4u + base, top), plane);
+          if constexpr (SEMB_CHECKED) {
+            const int i0 = soff - P.tau - 0x4B000000;
+            if ((valid >> (2 * pr)) & 1) report_window(P.status, __float_as_int(y.x) + i0, W, src_at(c)[e], tg.cdp, t0);
+            if ((valid >> (2 * pr + 1)) & 1)
+              report_window(P.status, __float_as_int(y.y) + i0, W, src_at(c)[e], tg.cdp, t0);
+          }
+          float2 s0 = make_float2(lds32(ax), lds32(ay));
+#pragma unroll
+          for (int j = 0; j < W; ++j) {
+            const float2 s1 = make_float2(lds32(ax + 4u * (j + 1)), lds32(ay + 4u * (j + 1)));
+            const float2 d = __ffma2_rn(s0, make_float2(-1.f, -1.f), s1);
+            const float2 v = __ffma2_rn(d, x, s0);
+            inum[j][pr] = __fadd2_rn(inum[j][pr], v);
+            iden[pr] = __ffma2_rn(v, v, iden[pr]);
+            if (pr == CS / 2) ms.h = (CS & 1) ? fmaf(d.y, d.y, ms.h) : fmaf(d.x, d.x, ms.h);
+            s0 = s1;
+          }
+        }
+        continue;
+      }
       bool single = true;
-      if (meta->raw[e]) {   // narrow
+      if (kind == 1) {   // narrow
         const float q = fmaf(cb, g.y, q0);
         const float t = sqrt_fast(q), ti = rsqrt_fast(q);   // NaN, or infinite: neither in nor out
         const float y = __fadd_rz(t, 8388608.0f);
         const float x = t - (y - 8388608.0f);
         const float k1 = (hdB * g.y) * ti;
         // the run stays within h samples of t, rounding included
-        const float h = fmaf(fabsf(k1), rmax, fmaf(4e-6f, (float)P.ns, 0.01f));
+        const float h = fmaf(k1, rmax, fmaf(4e-6f, (float)P.ns, 0.01f));
         const bool in = t - h >= (float)P.tau && t + h < (float)(P.ns - P.tau - 1) && h < 0.5f;
         const bool out = t + h < (float)P.tau || t - h >= (float)(P.ns - P.tau - 1);
-        const bool cross = fmaf(fabsf(k1), rmax, fabsf(x - 0.5f)) >= 0.5f;
-        const bool mom = in && !cross;
-        single = !mom && !out;
-        if (__any_sync(0xffffffffu, mom)) {
-          const uint32_t a = mom ? min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top) : top;
-          const float km = mom ? k1 : 0.f;
-          ms.add(a, mom ? x : 0.f, km, mom ? (k1 * k1) * ti : 0.f);
+        single = !in && !out;
+        if (__any_sync(0xffffffffu, in)) {
+          const uint32_t a = in ? min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top) : top;
+          ms.template add<true>(a, in ? x : 0.f, in ? k1 : 0.f, in ? (k1 * k1) * ti : 0.f);
+        }
+        if (in) {
+          const uint32_t up = x + k1 * rmax >= 1.0f ? 1u << (e & 31) : 0u, dn = x < k1 * rmax ? 1u << (e & 31) : 0u;
+#pragma unroll
+          for (int b = 0; b < kMaxChunk / 32; ++b)
+            if (e >> 5 == b) {
+              up_mask[b] |= up;
+              dn_mask[b] |= dn;
+            }
         }
         if (out) {
           miss2 |= miss1;
@@ -585,42 +587,127 @@ __global__ void __launch_bounds__(kFilterNT, 1) semb_filter_kernel(FilterParams 
         // t^2 within dq of the record's ends may be in range or not in the direct
         // kernels' rounding: such an item is kept whatever its sums
         const float dq = 9.5e-7f * fmaf(u, u, fmaf(P.bmax, g.y, fabsf(cc) * g.z));
+        const float qc = fmaf(cb, g.y, q0), qs = P.dB * g.y;
+        uint32_t off_now = 0, near_end = 0;   // items out of range, items within dq of an end
 #pragma unroll
-        for (int r = 0; r < RC; ++r) {
-          if (!((valid >> r) & 1)) continue;
-          const float q = fmaf(fmaf((float)(r - CS), P.dB, cb), g.y, q0);
-          const float t = sqrt_fast(q);   // NaN below 0: out of range
-          const float y = __fadd_rz(t, 8388608.0f);
-          const int rel = __float_as_int(y) - (0x4B000000 + P.tau);   // it - tau
-          const bool ok = single && (unsigned)rel <= span;
-          const float x = ok ? t - (y - 8388608.0f) : 0.0f;
-          const unsigned idx = min(ok ? (unsigned)(soff + rel) : (unsigned)P.cap, (unsigned)P.cap);
-          if constexpr (SEMB_CHECKED) {
-            if (ok) report_window(P.status, soff + rel, W, src_at(c)[e], tg.cdp, t0);
+        for (int pr = 0; pr < RP; ++pr) {
+          const float2 rr = make_float2((float)(2 * pr - CS), (float)(2 * pr + 1 - CS));
+          const float2 q = __ffma2_rn(rr, make_float2(qs, qs), make_float2(qc, qc));
+          const float2 t = make_float2(sqrt_fast(q.x), sqrt_fast(q.y));   // NaN below 0: out of range
+          const float2 y = __fadd2_rz(t, make_float2(8388608.0f, 8388608.0f));
+          float2 x = __ffma2_rn(__fadd2_rn(y, make_float2(-8388608.0f, -8388608.0f)), make_float2(-1.f, -1.f), t);
+          const int relx = __float_as_int(y.x) - (0x4B000000 + P.tau);   // it - tau
+          const int rely = __float_as_int(y.y) - (0x4B000000 + P.tau);
+          const bool okx = single && ((valid >> (2 * pr)) & 1) && (unsigned)relx <= span;
+          const bool oky = single && ((valid >> (2 * pr + 1)) & 1) && (unsigned)rely <= span;
+          if (!okx) {
+            x.x = 0.f;
+            off_now |= 1u << (2 * pr);
           }
-          float s[W + 1];
-#pragma unroll
-          for (int j = 0; j <= W; ++j) s[j] = lds32(plane + 4u * (idx + j));
-          float den = 0.f;
+          if (!oky) {
+            x.y = 0.f;
+            off_now |= 1u << (2 * pr + 1);
+          }
+          if (fabsf(q.x - q_lo) <= dq || fabsf(q.x - q_hi) <= dq) near_end |= 1u << (2 * pr);
+          if (fabsf(q.y - q_lo) <= dq || fabsf(q.y - q_hi) <= dq) near_end |= 1u << (2 * pr + 1);
+          if constexpr (SEMB_CHECKED) {
+            if (okx) report_window(P.status, soff + relx, W, src_at(c)[e], tg.cdp, t0);
+            if (oky) report_window(P.status, soff + rely, W, src_at(c)[e], tg.cdp, t0);
+          }
+          const uint32_t ax = okx ? min(plane + 4u * (uint32_t)(soff + relx), top) : top;
+          const uint32_t ay = oky ? min(plane + 4u * (uint32_t)(soff + rely), top) : top;
+          float2 s0 = make_float2(lds32(ax), lds32(ay));
 #pragma unroll
           for (int j = 0; j < W; ++j) {
-            const float d = s[j + 1] - s[j];
-            const float v = fmaf(d, x, s[j]);
-            if (r & 1) inum[j][r >> 1].y += v;
-            else inum[j][r >> 1].x += v;
-            den = fmaf(v, v, den);
-            if (r == CS) ms.h = fmaf(d, d, ms.h);
-          }
-          if (r & 1) iden[r >> 1].y += den;
-          else iden[r >> 1].x += den;
-          if (single && (fabsf(q - q_lo) <= dq || fabsf(q - q_hi) <= dq)) {
-            unsure |= 1u << r;
-          } else if (single && !ok) {
-            miss2 |= miss1 & (1u << r);
-            miss1 |= 1u << r;
+            const float2 s1 = make_float2(lds32(ax + 4u * (j + 1)), lds32(ay + 4u * (j + 1)));
+            const float2 d = __ffma2_rn(s0, make_float2(-1.f, -1.f), s1);
+            const float2 v = __ffma2_rn(d, x, s0);
+            inum[j][pr] = __fadd2_rn(inum[j][pr], v);
+            iden[pr] = __ffma2_rn(v, v, iden[pr]);
+            if (pr == CS / 2) ms.h = (CS & 1) ? fmaf(d.y, d.y, ms.h) : fmaf(d.x, d.x, ms.h);
+            s0 = s1;
           }
         }
+        if (single) {
+          unsure |= near_end;
+          miss2 |= miss1 & off_now & ~near_end;
+          miss1 |= off_now & ~near_end;
+        }
       }
+    }
+    // crossings: each lane takes its next noted trace until none has one, first those above
+    // the centre (dB >= 0: items of the higher slots), then those below
+    auto crossings = [&](auto quad_c, auto up_c, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+      constexpr bool QUAD = decltype(quad_c)::value, UP = decltype(up_c)::value;
+      while (__any_sync(0xffffffffu, (m0 | m1 | m2 | m3) != 0)) {
+        const bool have = (m0 | m1 | m2 | m3) != 0;
+        int e = 0;
+        if (m0) {
+          e = __ffs(m0) - 1;
+          m0 &= m0 - 1;
+        } else if (m1) {
+          e = 31 + __ffs(m1);
+          m1 &= m1 - 1;
+        } else if (m2) {
+          e = 63 + __ffs(m2);
+          m2 &= m2 - 1;
+        } else if (m3) {
+          e = 95 + __ffs(m3);
+          m3 &= m3 - 1;
+        }
+        const float4 g = meta->geo[e];
+        const float u = fmaf(ca, g.x, T);
+        const float q = fmaf(cb, g.y, fmaf(u, u, cc * g.z));
+        const float t = sqrt_fast(q), ti = rsqrt_fast(q);
+        const float y = __fadd_rz(t, 8388608.0f);
+        const float x = t - (y - 8388608.0f);
+        const float k1 = (hdB * g.y) * ti;
+        // the boundary samples p_1 .. p_W with their neighbours p_0, p_W+1: the window
+        // itself for a crossing upwards, one sample earlier for one downwards; without a
+        // trace the zero block
+        const uint32_t a =
+            have ? min((__float_as_uint(y) + __float_as_uint(g.w)) * 4u + base0, top) - (UP ? 0u : 4u) : top;
+        if constexpr (SEMB_CHECKED) {
+          if (have)
+            report_window(P.status, __float_as_int(y) - 0x4B000000 - P.tau + __float_as_int(g.w) - (UP ? 0 : 1), W + 1,
+                          src_at(c)[e], tg.cdp, t0);
+        }
+        float p[W + 2];
+#pragma unroll
+        for (int j = 0; j < W + 2; ++j) p[j] = lds32(a + 4u * j);
+        // distance beyond the boundary z_r = z0 + a1 r + a2 r^2; beyond it sample j is
+        // p_j+1 + e_j z + c_j z with e_j the centre interval's slope along z
+        const float z0 = have ? (UP ? x - 1.0f : -x) : 0.f;
+        const float a1 = have ? (UP ? k1 : -k1) : 0.f;
+        const float a2 = QUAD && have ? (UP ? -0.5f : 0.5f) * ((k1 * k1) * ti) : 0.f;
+        float cj[W], q1 = 0.f, q2 = 0.f;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          const float dm = p[j + 1] - p[j], dp = p[j + 2] - p[j + 1];
+          cj[j] = dp - dm;
+          q1 = fmaf(cj[j], p[j + 1], q1);
+          q2 = fmaf(cj[j], fmaf(2.f, UP ? dm : -dp, cj[j]), q2);
+        }
+        const float2 z02 = make_float2(z0, z0), a12 = make_float2(a1, a1), a22 = make_float2(a2, a2);
+        const float2 q12 = make_float2(2.f * q1, 2.f * q1), q22 = make_float2(q2, q2);
+        // only the slots on that side of the centre
+#pragma unroll
+        for (int pr = UP ? (CS + 1) / 2 : 0; pr < (UP ? RP : (CS + 1) / 2); ++pr) {
+          const float2 rr = make_float2((float)(2 * pr - CS), (float)(2 * pr + 1 - CS));
+          float2 z = __ffma2_rn(rr, QUAD ? __ffma2_rn(rr, a22, a12) : a12, z02);
+          z = make_float2(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f));
+#pragma unroll
+          for (int j = 0; j < W; ++j) inum[j][pr] = __ffma2_rn(make_float2(cj[j], cj[j]), z, inum[j][pr]);
+          iden[pr] = __ffma2_rn(z, __ffma2_rn(z, q22, q12), iden[pr]);
+        }
+      }
+    };
+    if (quad) {
+      crossings(std::true_type{}, std::true_type{}, up_mask[0], up_mask[1], up_mask[2], up_mask[3]);
+      crossings(std::true_type{}, std::false_type{}, dn_mask[0], dn_mask[1], dn_mask[2], dn_mask[3]);
+    } else {
+      crossings(std::false_type{}, std::true_type{}, up_mask[0], up_mask[1], up_mask[2], up_mask[3]);
+      crossings(std::false_type{}, std::false_type{}, dn_mask[0], dn_mask[1], dn_mask[2], dn_mask[3]);
     }
     n_tot += n;
     // the plane and metadata of chunk c are no longer read by this warp

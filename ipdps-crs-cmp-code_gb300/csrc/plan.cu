@@ -51,9 +51,10 @@ int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, 
 int launch_repick(int w, const RepickParams& R, cudaStream_t st);
 int launch_crs_de(int w, const DeParams& R, cudaStream_t st);
 bool filter_exists(int form, int w, int brun, int pipe, int lay);
-size_t filter_smem(int form, int storage, int cap);
-int filter_prepare(int form, int w, int storage, size_t smem);
-int launch_filter(int form, int w, int storage, const FilterParams& F, int nwarps, int grid, size_t smem,
+int filter_shape(int w, int nb, int* rc, int* nt);
+size_t filter_smem(int form, int storage, int nt, int cap);
+int filter_prepare(int form, int w, int storage, int shape, size_t smem);
+int launch_filter(int form, int w, int storage, int shape, const FilterParams& F, int nwarps, int grid, size_t smem,
                   cudaStream_t st);
 int launch_refine(int form, int w, int lay, const RefineParams& R, cudaStream_t st);
 
@@ -66,7 +67,7 @@ namespace {
 // The filter in front of a direct CRS configuration (filter_kernel.cuh): its candidate
 // runs, passes, staging capacity and launch shape.
 struct FilterCfg {
-  int nwarps = 0, npass = 0, cap = 0, nbp = 0, z0 = 0, lay = 0;
+  int shape = 0, rc = 0, nwarps = 0, npass = 0, cap = 0, nbp = 0, z0 = 0, lay = 0;
   size_t smem = 0;
   float dB = 0.f, hbr = 0.f, bmax = 0.f;
   float4* d_cand = nullptr;
@@ -434,19 +435,22 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   const semb_params& p = pl->p;
   const int form = p.mode == SEMB_PLAIN_F32 ? FORM_PLAIN : FORM_FAST;
   if (p.method != SEMB_CRS || p.ngen > 0 || p.nb < 2 || !filter_exists(form, pl->w, brun, pipe, lay)) return SEMB_OK;
-  const int rc = filter_rc(pl->w), cs = (rc - 1) / 2;
+  int rc = 0, nt = 0;
+  const int shape = filter_shape(pl->w, p.nb, &rc, &nt), cs = (rc - 1) / 2;
   const int nruns = (p.nb + rc - 1) / rc;
   const int64_t total = (int64_t)p.na * p.nc * nruns;
-  // Warp instructions per aperture trace of one task (32 t0): the direct kernels evaluate
-  // every candidate (about 21 instructions batched, 56 plain), the filter every run (90
-  // with its crossings), the refine 32 t0.  Below the line the filter does not pay: a
-  // 9 x 13 x 5 grid with w = 5 took 3.34 ms with it and 3.42 without, 7 x 21 x 7 with few
-  // tasks 2.4 and 1.3.
-  const double direct = (form == FORM_PLAIN ? 56.0 : 21.0) * (double)pl->ncand;
-  const double filtered = 90.0 * (double)total + (form == FORM_PLAIN ? 45.0 : 95.0) * 32.0;
+  // Scheduler cycles per aperture trace of one task (32 t0), from whole searches on GB300:
+  // a candidate of the direct kernels takes about 25 (batched) or 73 (plain), a run of the
+  // filter about 100 and 3.5 per slot, the refine 3500 (plain) or 8600.  Below the line the
+  // filter does not pay: a 9 x 13 x 5 grid (w = 5) took 2.6 ms with it and 3.4 without, a
+  // 7 x 21 x 7 grid with little more than one task per SM 1.5 and 1.3.
+  const double direct = (form == FORM_PLAIN ? 73.0 : 25.0 + (pl->w == 5 ? 8.0 : 0.0)) * (double)pl->ncand;
+  const double filtered = (100.0 + 3.5 * rc) * (double)total + (form == FORM_PLAIN ? 3500.0 : 8600.0);
   if (filtered > 0.9 * direct) return SEMB_OK;
   // each (A, C) group's B values cut into the fewest runs of at most rc, of equal length
-  // give or take one, each run's middle value in slot cs; padding repeats the run's ends
+  // give or take one, each run's middle value in slot cs, B ascending with the slot; padding
+  // repeats the run's ends
+  const bool down = p.b1 < p.b0;
   std::vector<int> slots;
   slots.reserve((size_t)total * rc);
   int widest = 0;
@@ -457,19 +461,22 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
       widest = std::max(widest, n - 1 - mid);
       for (int q = 0; q < rc; ++q) {
         const int i = q - cs + mid, ic = std::min(std::max(i, 0), n - 1);
-        slots.push_back(i == ic ? pl->order[g0 + b0 + i] : -1 - pl->order[g0 + b0 + ic]);
+        const int gi = pl->order[g0 + b0 + (down ? n - 1 - ic : ic)];
+        slots.push_back(i == ic ? gi : -1 - gi);
       }
     }
-  const double dB = (p.b1 - p.b0) * (1.0 / (double)p.nb) * (pl->idt64 * pl->idt64);
-  const double hbr = 0.5 * std::fabs(dB) * widest * (1.0 + 1e-6);
+  const double dB = std::fabs(p.b1 - p.b0) * (1.0 / (double)p.nb) * (pl->idt64 * pl->idt64);
+  const double hbr = 0.5 * dB * widest * (1.0 + 1e-6);
   // the widest trace of the aperture must expand from a quarter of the record on
   const double tq = 0.25 * pl->ns, h2 = hbr * (double)p.apm * (double)p.apm;
   if (!(h2 <= std::min(0.49, 0.0048 * tq) * tq)) return SEMB_OK;
 
   FilterCfg f;
+  f.shape = shape;
+  f.rc = rc;
   // warps in fours (one per scheduler); the most whose padding stays within 4%
   int64_t best_tot = INT64_MAX;
-  for (int nw = kFilterNT / 32; nw >= 4; nw -= 4) {
+  for (int nw = nt / 32; nw >= 4; nw -= 4) {
     const int64_t tot = (total + nw - 1) / nw * nw;
     if (tot < best_tot) {
       best_tot = tot;
@@ -480,10 +487,10 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   f.npass = (int)((total + f.nwarps - 1) / f.nwarps);
   const int store = form == FORM_PLAIN ? SEMB_STORE_F32 : p.storage;
   int cap = 16384;
-  while (cap > 64 && filter_smem(form, store, cap) > 226 * 1024) cap -= 64;
+  while (cap > 64 && filter_smem(form, store, nt, cap) > 226 * 1024) cap -= 64;
   if (cap < (int)pl->pitch + 16) return SEMB_OK;   // a window may span the whole record
   f.cap = cap;
-  f.smem = filter_smem(form, store, cap);
+  f.smem = filter_smem(form, store, nt, cap);
   f.dB = (float)dB;
   f.hbr = (float)hbr;
   f.bmax = (float)(std::max(std::fabs(p.b0), std::fabs(p.b1)) * (pl->idt64 * pl->idt64));
@@ -515,7 +522,7 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(f.d_pass_bounds, bounds.data(), bounds.size() * 4, cudaMemcpyHostToDevice, pl->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(pl->stream);
-  int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, f.smem) : SEMB_OK;
+  int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, shape, f.smem) : SEMB_OK;
   if (e != cudaSuccess || rc_prep != SEMB_OK) {
     dev_free(f.d_cand);
     dev_free(f.d_pass_bounds);
@@ -1277,7 +1284,7 @@ int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int n
     F.k.cand = f->d_cand;
     F.k.pass_bounds = f->d_pass_bounds;
     F.k.npass = f->npass;
-    F.k.cpp = f->nwarps * filter_rc(pl->w);
+    F.k.cpp = f->nwarps * f->rc;
     F.k.cap = f->cap;
     F.k.dB = f->dB;
     F.k.hbr = f->hbr;
@@ -1290,12 +1297,13 @@ int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int n
     F.fb_tasks = pl->d_fb_tasks;
     F.fb_count = pl->d_fb_count;
     F.kappa = form == FORM_PLAIN ? 16.f : 8.f;
-    SEMB_TRY(launch_filter(form, pl->w, P.storage, F, f->nwarps, std::min(ntasks, pl->sms), f->smem, st));
+    SEMB_TRY(launch_filter(form, pl->w, P.storage, f->shape, F, f->nwarps, std::min(ntasks, pl->sms), f->smem, st));
     RefineParams R{};
     R.k = P;
     R.head = pl->d_head;
     R.pool = pl->d_pool;
     R.runs = f->d_cand;
+    R.rc = f->rc;
     R.tasks = tasks;
     R.ntasks = ntasks;
     R.na = p.na;

@@ -28,7 +28,8 @@ struct RefineParams {
   KParams k;              // the direct configuration: stores, apertures, passes, capacity, outputs
   const int2* head;       // the filter's output
   const int2* pool;
-  const float4* runs;     // the filter's candidate runs
+  const float4* runs;     // the filter's candidate runs, rc slots each
+  int rc;
   const int2* tasks;
   int ntasks;
   int na, nb, nc;
@@ -39,27 +40,27 @@ struct RefineParams {
 constexpr int kRefineLanes = 16;   // lanes per (CDP, t0): a warp takes 32 / kRefineLanes of them
 
 // The kept candidates of one item, dealt out to its lanes.
-template <int RC>
 struct Kept {
   const int2* e = nullptr;
-  int n = 0, total = 0;
+  int n = 0, total = 0, rc = 0;
 
   // false: the item fell back
   __device__ __forceinline__ bool load(const RefineParams& R, int64_t item) {
     const int2 h = __ldg(R.head + item);
     if (h.y < 0) return false;
     e = R.pool + h.x;
+    rc = R.rc;
     n = h.y;
     for (int q = 0; q < n; ++q) total += __popc(__ldg(&e[q].y));
     return true;
   }
-  // slot index (run * RC + slot) of candidate i, -1 past the end
+  // slot index (run * rc + slot) of candidate i, -1 past the end
   __device__ __forceinline__ int at(int i) const {
     if (i >= total) return -1;
     for (int q = 0; q < n; ++q) {
       const int2 v = __ldg(e + q);
       const int c = __popc(v.y);
-      if (i < c) return v.x * RC + (int)__fns((unsigned)v.y, 0, i + 1);
+      if (i < c) return v.x * rc + (int)__fns((unsigned)v.y, 0, i + 1);
       i -= c;
     }
     return -1;
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(256) k_refine_plain(RefineParams R) {
   const int2 td = R.tasks[unit / PER];
   const int cdp = td.x, t0 = td.y + (int)(unit % PER) * (32 / G) + lane / G;
   const int64_t item = (int64_t)cdp * P.ns + min(t0, P.ns - 1);
-  Kept<filter_rc(W)> kept;
+  Kept kept;
   const bool live = t0 < P.ns && kept.load(R, item);
   const int most = __reduce_max_sync(0xffffffffu, live ? kept.total : 0);
   if (!__any_sync(0xffffffffu, live)) return;
@@ -223,7 +224,7 @@ __global__ void __launch_bounds__(256) k_refine_fast(RefineParams R) {
   const int2 td = R.tasks[unit / PER];
   const int cdp = td.x, t0 = td.y + (int)(unit % PER) * (32 / G) + lane / G;
   const int64_t item = (int64_t)cdp * P.ns + min(t0, P.ns - 1);
-  Kept<filter_rc(W)> kept;
+  Kept kept;
   const bool live = t0 < P.ns && kept.load(R, item);
   const int most = __reduce_max_sync(0xffffffffu, live ? kept.total : 0);
   if (!__any_sync(0xffffffffu, live)) return;

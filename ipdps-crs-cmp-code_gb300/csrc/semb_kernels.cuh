@@ -285,6 +285,8 @@ struct ChunkMeta {
                            // [kMaxChunk - (n - n_in), kMaxChunk).  Plain form: n_in = n
   int consumed;            // aperture traces the chunk covers (entries + skipped)
   int bytes;               // bytes staged (TMA form)
+  int quad;                // semb_filter_kernel: some in-range entry needs the expansion's
+                           // second-order terms
 };
 
 constexpr size_t kMetaBytes = ((sizeof(ChunkMeta) + 127) / 128) * 128;
@@ -394,6 +396,13 @@ __device__ __forceinline__ bool moment_narrow(float h2, float smin) {
   return h2 <= fminf(0.49f, 0.0048f * smin) * smin;
 }
 
+// Whether the expansion's second-order term, at most h^2 / (2 t) samples for a half
+// spread h = h2 / t, is below 0.2 of a traveltime's rounding at the record's end, t 2^-24
+// with t = ns: then it is left out, within the filter's bounds.
+__device__ __forceinline__ bool moment_linear(float h2, float smin, float ns) {
+  return h2 * h2 <= 0.4f * 5.9604645e-8f * ns * (smin * smin) * smin;
+}
+
 // Warp 0: choose the entries of the next chunk starting at ap_pos and record, per
 // entry, its geometry, its buffer offset (minus the window start, so that an item
 // indexes with it - tau directly) and its source window (trace, first sample,
@@ -401,8 +410,9 @@ __device__ __forceinline__ bool moment_narrow(float h2, float smin) {
 // consumed without an entry.  meta->n counts entries, meta->consumed the aperture
 // traces the chunk covers.  Fast form: entries on which every item is in range go
 // to the front slots, the others to the back (entry_slot); MOM keeps only entries
-// whose B runs expand about their centre (moment_narrow) in front, and raw[] says which of
-// the others do.  Windows are aligned to ALIGN samples: 4 for FP32 bulk
+// whose B runs expand about their centre (moment_narrow) in front; raw[] is 1 for
+// the others that do, 2 for those that do not but have every item in range.  Windows are
+// aligned to ALIGN samples: 4 for FP32 bulk
 // copies (16 bytes), 8 for the fast form's raw windows.  Buffer units: floats
 // (plain) or one 16-byte entry per sample (fast).
 template <int METHOD, int FORM, bool MOM = false>
@@ -414,6 +424,7 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
   int n_in = 0;       // entries in the in-range part (front)
   int n_out = 0;      // other entries (back)
   int consumed = 0;   // aperture traces covered
+  [[maybe_unused]] bool quad = false;
   while (n_in + n_out + 32 <= kMaxChunk) {
     const int64_t k = ap_pos + consumed + lane;
     const bool have = k < ap_end;
@@ -424,14 +435,16 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
     int tr = 0;
     float sc = 1.0f;
     bool glob = false;
-    [[maybe_unused]] bool narrow = false;
+    [[maybe_unused]] int kind = 0;
+    [[maybe_unused]] bool linear = true;
     if (have) {
       g = P.ap_geo[k];
       float smin = 0.f;
       keep = trace_window<METHOD>(pb, g, T_lo, T_hi, P.idt, P.tau, P.ns, lo, hi, inr, smin);
       if constexpr (MOM) {
-        narrow = moment_narrow(P.hbr * fabsf(g.y), smin);
-        inr = inr && narrow;
+        linear = moment_linear(P.hbr * fabsf(g.y), smin, (float)P.ns);
+        kind = moment_narrow(P.hbr * fabsf(g.y), smin) ? 1 : inr ? 2 : 0;
+        inr = inr && kind == 1;
       }
       // a trace of the central CDP at zero midpoint distance whose sums the pass shares
       // over A and B (Z0 variants) is left out
@@ -473,10 +486,11 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
       g.w = __int_as_float(glob ? kGlobalEntry : off - lo);
       meta->geo[e] = g;
       meta->scale[e] = sc;
-      if constexpr (MOM) meta->raw[e] = narrow ? 1 : 0;
+      if constexpr (MOM) meta->raw[e] = kind;
       else meta->raw[e] = glob ? tr : off + 8 * rank;
       src[e] = make_int4(tr, lo, len, off);   // len 0: nothing to copy or convert
     }
+    if constexpr (MOM) quad = quad || __any_sync(0xffffffffu, take && front && !linear);
     const int nhave = __popc(__ballot_sync(0xffffffffu, have));
     base += stop > 0 ? __shfl_sync(0xffffffffu, incl, stop - 1) : 0;
     n_in += __popc(fr);
@@ -489,6 +503,7 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
     meta->n_in = n_in;
     meta->consumed = consumed;
     meta->bytes = base * 4;
+    if constexpr (MOM) meta->quad = quad ? 1 : 0;
   }
   __syncwarp();
 }

@@ -27,9 +27,11 @@ def _survey(nb, tau, ns, apm, b1=1e-7, ncdp=9, fold=9, na=3, nc=5, az=0.0, seed=
 
 # runs of one, full runs, one past a full run, several runs; odd records; every window;
 # a B range so wide that most traces leave the expansion; apertures of one CDP, where
-# every A and B ties and the lists overflow into the direct kernel; no valid item at all
+# every A and B ties and the lists overflow into the direct kernel; no valid item at all; B
+# descending with its index
 CASES = [(12, 1, 301, 50, 1e-7, 9), (13, 1, 256, 50, 1e-7, 9), (24, 2, 333, 75, 1e-7, 9), (25, 0, 290, 50, 1e-7, 9),
-         (9, 2, 331, 50, 1e-7, 9), (31, 1, 300, 50, 3e-6, 9), (21, 1, 300, 5, 1e-7, 3), (21, 1, 64, 50, 1e-7, 9)]
+         (9, 2, 331, 50, 1e-7, 9), (31, 1, 300, 50, 3e-6, 9), (21, 1, 300, 5, 1e-7, 3), (21, 1, 64, 50, 1e-7, 9),
+         (21, 1, 300, 50, -1e-7, 9), (15, 2, 300, 50, 1e-7, 9)]
 
 
 @pytest.mark.parametrize("nb,tau,ns,apm,b1,ncdp", CASES)
