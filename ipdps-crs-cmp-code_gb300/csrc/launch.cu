@@ -1,6 +1,8 @@
 // Kernel lookup and launch helpers shared by the plan.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.h"
 #include "plan_kernels.cuh"
 #include "search_inst.cuh"
@@ -35,6 +37,36 @@ int search_variant(int method, int form, int w, int v, int* rc, int* minb, int* 
 // Candidate slots of one (A, C) group's run of nb B values padded to a multiple of rc.
 static int brun_slots(int nb, int rc) { return (std::max(nb, 1) + rc - 1) / rc * rc; }
 
+// Launch shape of semb_plain_kernel for ncand candidates at rc per thread and at most
+// max_warps warps per SM: warps per CTA and CTAs per SM (several where one needs few
+// warps).  Returns its cost, time per aperture trace in candidates per lane: a pass of nw
+// warps takes its schedulers ceil(nw / 4) warps' time each, and not less than `few` warps'
+// (with fewer, the latency of a warp's own chain shows).
+double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas) {
+  const double few = rc == 8 ? 2.5 : 4.0;
+  double best = 1e300;
+  for (int nw = max_warps; nw >= 4; --nw) {
+    const int npass = (ncand + nw * rc - 1) / (nw * rc), k = std::min(4, max_warps / nw);
+    const double cost = (double)npass * rc * std::max((double)((nw * k + 3) / 4), few) / k;
+    if (cost < best) {
+      best = cost;
+      *nwarps = nw;
+      *ctas = k;
+    }
+  }
+  return best;
+}
+
+// Plain form, windows up to 5: 8 candidates per thread (variant 0) unless 4 (variant 1)
+// use the warps better.  Measured, variant 0 / 1 / the two-barrier kernel (ms): 256
+// candidates, w = 5: 8.66 / 9.21 / 11.44; 200, w = 3: 3.24 / 3.19 / 5.03; 101, w = 3: 1.86 /
+// 1.74 / 2.37; 90, w = 5: 1.98 / 2.09 / 2.57; 64, w = 3: 1.96 / 2.19 / 2.42; 33, w = 1: 0.50 /
+// 0.44 / 0.80.
+static int plain_variant(int ncand) {
+  int nw, k;
+  return plain_shape(ncand, 4, 26, &nw, &k) < 0.97 * plain_shape(ncand, 8, 16, &nw, &k) ? 1 : 0;
+}
+
 // Variant a plan starts with (before any autotuning), the fastest measured on GB300
 // for the benchmark workloads of each window: for CRS the pipelined B-run kernel
 // (packed value/difference staging with a two-way trace unroll and the central traces'
@@ -46,8 +78,8 @@ static int brun_slots(int nb, int rc) { return (std::max(nb, 1) + rc - 1) / rc *
 // slot the two run at the same speed).  fallback_variant() is the one to use where the
 // default does not fit the plan (a grid whose passes span more C values than the
 // central-trace sharing takes).
-int default_variant(int method, int form, int w, int nb) {
-  if (form != FORM_FAST) return 0;
+int default_variant(int method, int form, int w, int nb, int ncand) {
+  if (form != FORM_FAST) return w <= 5 ? plain_variant(ncand) : 0;
   if (method == METHOD_CRS && w == 3) return brun_slots(nb, 8) < brun_slots(nb, 7) ? 33 : 30;
   if (method == METHOD_CRS && w <= 5) return 14;
   if (method == METHOD_CMP && w == 3) return 8;
@@ -56,6 +88,7 @@ int default_variant(int method, int form, int w, int nb) {
 }
 
 int fallback_variant(int method, int form, int w, int nb) {
+  if (form != FORM_FAST) return w <= 5 ? 2 : 0;
   if (form == FORM_FAST && method == METHOD_CRS && w == 3) return brun_slots(nb, 8) < brun_slots(nb, 7) ? 32 : 13;
   return 0;
 }

@@ -19,9 +19,10 @@
 #include <vector>
 
 #include "common.h"
-#include "refine_kernel.cuh"
 #include "pipe_kernel.cuh"
+#include "plain_kernel.cuh"
 #include "plan_kernels.cuh"
+#include "refine_kernel.cuh"
 #include "semb_kernels.cuh"
 
 namespace semb {
@@ -39,7 +40,8 @@ constexpr int kBucketSplits = 3;
 constexpr int kBucketAp[kBucketSplits] = {1024, 384, 128};
 static_assert(kBucketSplits + 1 <= kMaxBuckets, "bucket table");
 int search_occupancy(int method, int form, int w, int variant, int nwarps, size_t smem, int* ctas_per_sm);
-int default_variant(int method, int form, int w, int nb);
+int default_variant(int method, int form, int w, int nb, int ncand);
+double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas);
 int fallback_variant(int method, int form, int w, int nb);
 int grid_neighbours(int ncdps, const float* d_fmx, const float* d_fmy, int apm, int64_t* d_off, int32_t** d_list,
                     int64_t* n_out, cudaStream_t st);
@@ -78,6 +80,7 @@ struct FilterCfg {
 // parameter bounds, staging capacity, shared memory and residency.
 struct KernelCfg {
   int variant = -1, rc = 0, minb = 0, nwarps = 0, cpp = 0, npass = 0, cap = 0, occ = 0;
+  bool queue = false;   // persistent CTAs over the work queue (else one CTA per task)
   size_t smem = 0;
   float4* d_cand = nullptr;
   float* d_pass_bounds = nullptr;
@@ -583,6 +586,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
       best_nw = nw;
     }
   }
+  if (pipe == 3) plain_shape(nslots, rc, nt / 32, &best_nw, &minb);
   const int cpp = best_nw * rc;
   const int npass = (nslots + cpp - 1) / cpp;
   // Z0 variants: each pass's C indices (C is outermost in the search order, so they are
@@ -617,11 +621,16 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   // plan's stage_cap, which also bounds it from above).
   const bool small_stages = form == FORM_FAST && glob;
   const int store = (form == FORM_FAST) ? p.storage : SEMB_STORE_F32;
+  // the ring kernel's CTAs share the SM only where each still holds a whole trace's window
+  // in every plane
+  while (pipe == 3 && minb > 1 && plain_layout((int)pl->pitch + 16, nt).total > (227 * 1024) / (size_t)minb - 1024) --minb;
   const size_t budget = (227 * 1024) / minb - 1024;
   int cap = form == FORM_PLAIN ? 32768 : 8192;
   if (form == FORM_FAST && pl->stage_cap > 0) cap = std::min(cap, pl->stage_cap);
   auto smem_of = [&](int cp) {
-    return pipe ? pipe_layout(rc, cp, store, nt, lay, z0).total : smem_layout(form, rc, cp, store, nt, lay).total;
+    return pipe == 3 ? plain_layout(cp, nt).total
+           : pipe    ? pipe_layout(rc, cp, store, nt, lay, z0).total
+                     : smem_layout(form, rc, cp, store, nt, lay).total;
   };
   if (lay == LAY_X3) cap = std::min(cap, kXPlane - kZeroSlots);
   while (cap > 64 && smem_of(cap) > budget) cap -= 64;
@@ -677,6 +686,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   c.cap = cap;
   c.smem = smem;
   c.occ = occ;
+  c.queue = form == FORM_FAST || pipe == 3;
   const int frc = attach_filter(pl, brun, pipe, lay, z0, rc, c);
   if (frc != SEMB_OK) {
     free_cfg(c);
@@ -690,7 +700,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
 
 int bucket_grid(const semb_plan* pl, const Bucket& b) {
   const int n = b.end - b.begin;
-  return pl->p.mode == SEMB_PLAIN_F32 ? n : std::min(n, pl->sms * b.cfg.occ);
+  return b.cfg.queue ? std::min(n, pl->sms * b.cfg.occ) : n;
 }
 
 // The bucket that holds most of the search work (its variant is the one reported).
@@ -1204,7 +1214,7 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   for (int i = 0; i < g->ncdps; ++i) pl->aperture[i] = (int32_t)(ap_off[i + 1] - ap_off[i]);
 
   // the default variant of this method and window; variant 0 where it does not fit
-  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb)) != SEMB_OK &&
+  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand)) != SEMB_OK &&
       set_all(pl, fallback_variant(p.method, form, pl->w, p.nb)) != SEMB_OK)
     SEMB_TRY(set_all(pl, 0));
   // streamed: the other chunks' copies, after the set-up's own small copies
@@ -1270,7 +1280,7 @@ KParams make_kparams_cfg(semb_plan* pl, const KernelCfg& cfg, const int2* tasks,
 }
 
 // The search of tasks[0, ntasks) with configuration cfg on stream st, work-queue head
-// `counter` (zeroed by the caller; the plain form has none): the direct kernel, or the filter, the refine of what it kept and
+// `counter` (zeroed by the caller): the direct kernel, or the filter, the refine of what it kept and
 // the direct kernel on the tasks whose lists overflowed.  grid: the direct kernel's.
 int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int ntasks, int grid, int* counter,
                    cudaStream_t st, int* launches) {
@@ -1391,7 +1401,7 @@ int enqueue_run(semb_plan* pl, bool timed) {
     pl->stats.kernel_launches = launches;
     return SEMB_OK;
   }
-  if (form == FORM_FAST) SEMB_CUDA(cudaMemsetAsync(pl->d_counter, 0, kMaxBuckets * sizeof(int), st));
+  SEMB_CUDA(cudaMemsetAsync(pl->d_counter, 0, kMaxBuckets * sizeof(int), st));
   if (timed) SEMB_CUDA(cudaEventRecord(pl->ev[1], st));
   // neighbouring buckets on the same variant (same launch configuration) run as one
   // launch over their tasks, longest aperture first, on the first one's queue head
@@ -1857,7 +1867,7 @@ int semb_plan_autotune(semb_plan* pl, int32_t* chosen, double* ms_of_variant) {
         fits[v] = 0;
         continue;
       }
-      const int grid = form == FORM_PLAIN ? S : std::min(S, pl->sms * guard.trial.occ);
+      const int grid = guard.trial.queue ? std::min(S, pl->sms * guard.trial.occ) : S;
       float ms = 1e30f;
       for (int rep = 0; rep < 3; ++rep) {
         SEMB_CUDA(cudaMemsetAsync(pl->d_counter, 0, sizeof(int), st));

@@ -21,6 +21,7 @@
 
 #include "common.h"
 #include "pipe_kernel.cuh"
+#include "plain_kernel.cuh"
 #include "semb_kernels.cuh"
 
 namespace semb {
@@ -31,7 +32,7 @@ struct SearchEntry {
   int minb;
   int brun;   // candidates laid out as B runs of RC (CRS)
   int nt;     // threads per CTA
-  int pipe;   // 1: semb_pipe_kernel (decoupled staging ring), 0: semb_search_kernel
+  int pipe;   // 1: semb_pipe_kernel (decoupled staging ring), 3: semb_plain_kernel, 0: semb_search_kernel
   int lay;    // staging layout (LAY_*)
   int glob;   // 1: stages may be smaller than a trace (long windows read global memory)
   int z0;     // 1: the central traces' sums are shared over A and B (semb_pipe_kernel Z0)
@@ -59,27 +60,37 @@ SearchEntry pipe_entry() {
           LAY, GLOB ? 1 : 0, Z0 ? 1 : 0};
 }
 
-// Plain form: one variant per window.
+// Plain form: windows up to 5 in the ring kernel, with 8 candidates per thread in up to 16
+// warps (variant 0) or 4 in up to 26 (variant 1, for candidate counts that leave whole
+// warps idle in 8s; plain_variant() in launch.cu); wider windows, and records too long for
+// three planes (variant 2), in the two-barrier kernel.
 template <int METHOD, int W>
-SearchEntry plain_entry() {
-  constexpr int RC = W <= 5 ? 8 : W == 7 ? 6 : W <= 11 ? 4 : W == 13 ? 3 : 2;
-  return entry<METHOD, FORM_PLAIN, W, RC, 2>();
+SearchEntry plain_entry(int variant) {
+  if constexpr (W <= 5) {
+    if (variant == 2) return entry<METHOD, FORM_PLAIN, W, 8, 2>();
+    if (variant == 1) return {(const void*)semb_plain_kernel<METHOD, W, 4, 832>, 4, 1, 0, 832, 3, LAY_QUAD, 0, 0};
+    return {(const void*)semb_plain_kernel<METHOD, W, 8, 512>, 8, 1, 0, 512, 3, LAY_QUAD, 0, 0};
+  } else {
+    constexpr int RC = W == 7 ? 6 : W <= 11 ? 4 : W == 13 ? 3 : 2;
+    if (variant != 0) return {nullptr, 0, 0, 0, 0, 0, 0, 0, 0};
+    return entry<METHOD, FORM_PLAIN, W, RC, 2>();
+  }
 }
 
 template <int METHOD, int FORM>
 SearchEntry search_entry(int w, int variant) {
   if constexpr (FORM == FORM_PLAIN) {
-    if (variant != 0) return {nullptr, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (variant > 2) return {nullptr, 0, 0, 0, 0, 0, 0, 0, 0};
     switch (w) {
-      case 1: return plain_entry<METHOD, 1>();
-      case 3: return plain_entry<METHOD, 3>();
-      case 5: return plain_entry<METHOD, 5>();
+      case 1: return plain_entry<METHOD, 1>(variant);
+      case 3: return plain_entry<METHOD, 3>(variant);
+      case 5: return plain_entry<METHOD, 5>(variant);
 #if SEMB_WIDE_WINDOWS
-      case 7: return plain_entry<METHOD, 7>();
-      case 9: return plain_entry<METHOD, 9>();
-      case 11: return plain_entry<METHOD, 11>();
-      case 13: return plain_entry<METHOD, 13>();
-      case 15: return plain_entry<METHOD, 15>();
+      case 7: return plain_entry<METHOD, 7>(variant);
+      case 9: return plain_entry<METHOD, 9>(variant);
+      case 11: return plain_entry<METHOD, 11>(variant);
+      case 13: return plain_entry<METHOD, 13>(variant);
+      case 15: return plain_entry<METHOD, 15>(variant);
 #endif
       default: return {nullptr, 0, 0, 0, 0, 0, 0, 0, 0};
     }

@@ -276,7 +276,7 @@ __host__ __device__ constexpr int lay_stage_bytes(int lay) { return lay_has_side
 struct ChunkMeta {
   float4 geo[kMaxChunk];   // (|dm|, dm^2, h, soff as int bits)
   float scale[kMaxChunk];  // fast form: per-trace scale of the 16-bit store
-  int raw[kMaxChunk];      // fast form: start of the entry's raw window (samples):
+  int raw[kMaxChunk];      // plain form: 1 where every item is in range; fast form: start of the entry's raw window (samples):
                            // its buffer offset + 8 x its rank in aperture order;
                            // the trace index for a kGlobalEntry entry
   int n;                   // entries in this chunk
@@ -487,6 +487,7 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
       meta->geo[e] = g;
       meta->scale[e] = sc;
       if constexpr (MOM) meta->raw[e] = kind;
+      else if constexpr (FORM == FORM_PLAIN) meta->raw[e] = inr ? 1 : 0;
       else meta->raw[e] = glob ? tr : off + 8 * rank;
       src[e] = make_int4(tr, lo, len, off);   // len 0: nothing to copy or convert
     }
