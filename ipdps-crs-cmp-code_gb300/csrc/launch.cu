@@ -5,6 +5,7 @@
 
 #include "common.h"
 #include "plan_kernels.cuh"
+#include "repick_ff.cuh"
 #include "search_inst.cuh"
 
 namespace semb {
@@ -123,10 +124,18 @@ int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, 
   return SEMB_OK;
 }
 
-int launch_repick(int w, const RepickParams& R, cudaStream_t st) {
+// Items per warp: 32, so that one warp screens 32 consecutive items with one load each, but
+// fewer where that would leave the GPU's warps without work, as the near ties of a warp's
+// items run one after the other: 64 warps' worth of items per SM for CRS, most of whose items
+// are near ties (24 CDPs x 601 samples, w = 5: 3.2 ms at 32 per warp in FP64; 0.23 so, in
+// pairs of FP32 numbers), 8 for CMP, where 1% are and the screening of the others counts (75 x
+// 751, w = 11: 2% of the whole pass).
+int launch_repick(int w, RepickParams R, int sms, cudaStream_t st) {
   const int64_t items = R.item_end - R.item0;
   if (items <= 0) return SEMB_OK;
-  const int grid = (int)((items + 255) / 256);   // 32 items per warp, 8 warps per CTA
+  R.per_warp = 32;
+  while (R.per_warp > 1 && items < (int64_t)sms * (R.method == METHOD_CRS ? 64 : 8) * R.per_warp) R.per_warp /= 2;
+  const int grid = (int)((items + 8 * R.per_warp - 1) / (8 * R.per_warp));   // 8 warps per CTA
   switch (w) {
     case 1: k_repick<1><<<grid, 256, 0, st>>>(R); break;
     case 3: k_repick<3><<<grid, 256, 0, st>>>(R); break;

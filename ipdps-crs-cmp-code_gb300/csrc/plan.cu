@@ -50,7 +50,7 @@ constexpr int kGridNeighbours = 2048;
 // smallest automatic staging capacity of the batched form (samples per chunk)
 constexpr int kMinStage = 512;
 int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, float c, float* out, cudaStream_t st);
-int launch_repick(int w, const RepickParams& R, cudaStream_t st);
+int launch_repick(int w, RepickParams R, int sms, cudaStream_t st);
 int launch_crs_de(int w, const DeParams& R, cudaStream_t st);
 bool filter_exists(int form, int w, int brun, int pipe, int lay);
 int filter_shape(int w, int nb, int* rc, int* nt);
@@ -134,6 +134,7 @@ struct semb_plan {
   int32_t* d_ap_tr = nullptr;
   float4* d_ap_geo = nullptr;
   Geo64* d_ap_geo64 = nullptr;
+  float4* d_ap_ff = nullptr;   // CRS, batched: the double geometry as pairs of floats
   int64_t* d_nbr_off = nullptr;
   int32_t* d_nbr = nullptr;
   double* d_cand64 = nullptr;
@@ -293,6 +294,7 @@ void free_data(semb_plan* pl, bool keep_reusable = false) {
   release(pl->d_ap_tr);
   release(pl->d_ap_geo);
   release(pl->d_ap_geo64);
+  release(pl->d_ap_ff);
   release(pl->d_nbr_off);
   release(pl->d_nbr);
   for (Bucket& b : pl->buckets) free_cfg(b.cfg);
@@ -1045,12 +1047,18 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   SEMB_TRY(dev_reuse(pl, &pl->d_ap_tr, pl->nap));
   SEMB_TRY(dev_reuse(pl, &pl->d_ap_geo, pl->nap));
   SEMB_TRY(dev_reuse(pl, &pl->d_ap_geo64, pl->nap));
+  // the re-pick's geometry in pairs of floats (the extra attributes take the FP64 values);
+  // without the memory for it the re-pick is FP64 throughout
+  const bool ff = p.method == SEMB_CRS && p.mode == SEMB_BATCHED && p.repick != SEMB_REPICK_OFF && !p.attrs &&
+                  dev_reuse(pl, &pl->d_ap_ff, 2 * (size_t)pl->nap) == SEMB_OK;
+  if (!ff) cudaGetLastError();
   // azimuth direction for the signed midpoint displacement (SEMB_DM_SIGNED)
   const double az = p.azimuth * 3.14159265358979323846 / 180.0;
   const double cos_d = std::cos(az), sin_d = std::sin(az);
   k_aperture_fill<<<(g->ncdps + 7) / 8, 256, 0, st>>>(g->ncdps, p.method, pl->d_nbr_off, pl->d_nbr, d_cdp_end,
                                                        pl->d_ap_off, d_h32, d_mx32, d_my32, d_h64, d_mx64, d_my64,
                                                        pl->d_ap_tr, pl->d_ap_geo, pl->d_ap_geo64,
+                                                       ff ? pl->d_ap_ff : nullptr,
                                                        p.dm_mode == SEMB_DM_SIGNED ? 1 : 0, (float)cos_d,
                                                        (float)sin_d, cos_d, sin_d);
   SEMB_CUDA(cudaGetLastError());
@@ -1440,6 +1448,7 @@ int enqueue_repick(semb_plan* pl, cudaStream_t st, int cdp0, int cdp1, bool rese
     R.ap_off = pl->d_ap_off;
     R.ap_tr = pl->d_ap_tr;
     R.ap_geo64 = pl->d_ap_geo64;
+    R.ap_ff = p.attrs ? nullptr : pl->d_ap_ff;
     R.cand64 = pl->d_cand64;
     R.stt00 = pl->d_stt00;
     R.ncdps = pl->ncdps;
@@ -1461,7 +1470,7 @@ int enqueue_repick(semb_plan* pl, cudaStream_t st, int cdp0, int cdp1, bool rese
     R.item0 = (int64_t)cdp0 * pl->ns;
     R.item_end = (int64_t)cdp1 * pl->ns;
     if (reset_count) SEMB_CUDA(cudaMemsetAsync(pl->d_repicked, 0, sizeof(unsigned long long), st));
-    SEMB_TRY(launch_repick(pl->w, R, st));
+    SEMB_TRY(launch_repick(pl->w, R, pl->sms, st));
   }
   return SEMB_OK;
 }

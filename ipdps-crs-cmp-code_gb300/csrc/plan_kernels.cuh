@@ -155,6 +155,13 @@ static __global__ void k_aperture_count(int ncdps, const int64_t* __restrict__ n
   ap_cnt[i] = n;
 }
 
+// An entry's double geometry as pairs of floats (hi + lo): (m, m^2), (h, 0), for repick_ff.
+__device__ __forceinline__ void store_pairs(float4* out, const Geo64& g) {
+  const float m = (float)g.m, m2 = (float)g.m2, h = (float)g.h;
+  out[0] = make_float4(m, (float)(g.m - (double)m), m2, (float)(g.m2 - (double)m2));
+  out[1] = make_float4(h, (float)(g.h - (double)h), 0.f, 0.f);
+}
+
 // Aperture entries of CDP i (one warp per CDP): the traces of its neighbours in
 // list order, each trace's |dm|, dm^2 and h relative to the midpoint of CDP i's
 // first trace (CRS/OpenMP/src/main.cpp:179-204, 289-317), in float and in double.
@@ -167,7 +174,8 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
                                 const float* __restrict__ mx32, const float* __restrict__ my32,
                                 const double* __restrict__ h64, const double* __restrict__ mx64,
                                 const double* __restrict__ my64, int32_t* __restrict__ ap_tr,
-                                float4* __restrict__ ap_geo, Geo64* __restrict__ ap_geo64, int signed_dm,
+                                float4* __restrict__ ap_geo, Geo64* __restrict__ ap_geo64,
+                                float4* __restrict__ ap_ff, int signed_dm,
                                 float cos_f, float sin_f, double cos_d, double sin_d) {
   const int warps = blockDim.x >> 5;
   const int i = blockIdx.x * warps + (threadIdx.x >> 5);
@@ -189,14 +197,18 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
         ap_geo[e] = make_float4(m, __fmul_rn(m, m), h32[t], 0.f);
         const double dxd = __dsub_rn(mx64[t], cxd), dyd = __dsub_rn(my64[t], cyd);
         const double md = __dadd_rn(__dmul_rn(dxd, cos_d), __dmul_rn(dyd, sin_d));
-        ap_geo64[e] = Geo64{md, __dmul_rn(md, md), h64[t], 0.0};
+        const Geo64 g = {md, __dmul_rn(md, md), h64[t], 0.0};
+        ap_geo64[e] = g;
+        if (ap_ff) store_pairs(ap_ff + 2 * e, g);
       } else if (method == METHOD_CRS) {
         const float dx = __fsub_rn(mx32[t], cx), dy = __fsub_rn(my32[t], cy);
         const float m2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
         ap_geo[e] = make_float4(__fsqrt_rn(m2), m2, h32[t], 0.f);
         const double dxd = __dsub_rn(mx64[t], cxd), dyd = __dsub_rn(my64[t], cyd);
         const double m2d = __dadd_rn(__dmul_rn(dxd, dxd), __dmul_rn(dyd, dyd));
-        ap_geo64[e] = Geo64{__dsqrt_rn(m2d), m2d, h64[t], 0.0};
+        const Geo64 g = {__dsqrt_rn(m2d), m2d, h64[t], 0.0};
+        ap_geo64[e] = g;
+        if (ap_ff) store_pairs(ap_ff + 2 * e, g);
       } else {
         ap_geo[e] = make_float4(0.f, 0.f, h32[t], 0.f);
         ap_geo64[e] = Geo64{0.0, 0.0, h64[t], 0.0};
@@ -344,11 +356,14 @@ struct RepickParams {
   const int64_t* ap_off;
   const int32_t* ap_tr;
   const Geo64* ap_geo64;
+  const float4* ap_ff;         // the same as pairs of floats, two float4 per entry (CRS; null:
+                               // every near tie goes straight to FP64)
   const double* cand64;        // grid order: (a, b, c) x ncand, c in 1e6-scaled units
   const float* stt00;
   int ncdps, ns, tau, method, mode;
   int ncand;                   // candidates of the grid (full re-search of small items)
   int64_t item0, item_end;     // (CDP, t0) items cdp * ns + t0 of this launch
+  int per_warp;                // items per warp (1..32)
   double dt, idt;
   float gap;
   int32_t* ctr;
@@ -465,11 +480,17 @@ __device__ __forceinline__ void write_pick(const RepickParams& R, int64_t item, 
   }
 }
 
+template <int W>
+__device__ bool repick_ff(const RepickParams& R, int64_t e0, int64_t e1, int t0, const int (&ti)[kTopK], int lane, int& bi,
+                          float& bs, float& bk);
+
 // One near-tie item, all lanes of the warp: when the best two FP32 candidates are
 // closer than the near-tie band (repick_band: `gap`, wider for small apertures), or
 // always in mode 2, the top-4 are re-evaluated in FP64 with the reference's
 // double-precision arithmetic (CRS/OpenMP/src/main.cpp:209-267 with real = double)
-// on the FP32 samples, and the pick follows the FP64 values.  Small items whose
+// on the FP32 samples, and the pick follows the FP64 values (repick_ff gives the same
+// results from pairs of FP32 numbers where it can vouch for them; else this does).  Small
+// items whose
 // whole top-4 lies inside the band are re-searched over every candidate instead
 // (eval_f64_ordered, one candidate per lane), so that a candidate the FP32 ranking
 // put fifth or lower can still win as it does in FP64.
@@ -539,6 +560,21 @@ __device__ void repick_item(const RepickParams& R, const int64_t item, const int
     }
     if (lane == 0) atomicAdd(R.repicked, 1ull);
   } else if (redo) {
+    bool sure = false;
+    if constexpr (W <= 5) {
+      int fi;
+      float fs, fk;
+      // in pairs of FP32 numbers, where that determines the results
+      if (R.ap_ff && repick_ff<W>(R, e0, e1, t0, ti, lane, fi, fs, fk)) {
+        sure = true;
+        if (fi != 0x7fffffff) {
+          out_i = fi;
+          out_s = fs;
+          out_k = fk;
+        }
+      }
+    }
+    if (!sure) {
     // sums per candidate; the stack's linear sum is taken as the sum of the window
     // numerators at the end (the same quantity, summed in another order)
     double num[kTopK][W], den[kTopK];
@@ -630,23 +666,24 @@ __device__ void repick_item(const RepickParams& R, const int64_t item, const int
       for (int q = 0; q < kTopK; ++q)
         if (ti0[q] == bi) err = (float)fabs((double)ts[q] - bs);
     }
+    }
     if (lane == 0) atomicAdd(R.repicked, 1ull);
   }
   if (lane == 0) write_pick(R, item, cdp, none, out_i, out_s, out_k, err, ts, ti0);
 }
 
-// Final pick per (CDP, t0), 32 consecutive items per warp: each lane screens one
+// Final pick per (CDP, t0), R.per_warp consecutive items per warp: each lane screens one
 // item (no candidate above 0, or no near tie: the FP32 pick stands and the lane writes
 // it), then the warp takes the near-tie items one after the other (repick_item), all
 // lanes on one item's FP64 evaluation.
 template <int W>
-static __global__ void k_repick(RepickParams R) {
+static __global__ void __launch_bounds__(256, W <= 5 ? 2 : 1) k_repick(RepickParams R) {
   const int lane = threadIdx.x & 31;
-  const int64_t base = R.item0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+  const int64_t base = R.item0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R.per_warp;
   if (base >= R.item_end) return;
   const int64_t item = base + lane;
   bool redo = false;
-  if (item < R.item_end) {
+  if (lane < R.per_warp && item < R.item_end) {
     const int cdp = (int)(item / R.ns);
     float ts[kTopK], tk[kTopK];
     int ti[kTopK];

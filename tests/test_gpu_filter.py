@@ -88,3 +88,23 @@ def test_batched_filtered_search_agrees_with_the_direct_search(nb, tau, ns, apm,
     same = ctr == c0
     np.testing.assert_allclose(stk[same], k0[same], atol=2e-6, rtol=1e-5)
     assert np.mean(same) >= (0.99 if apm > 12 else 0.0)   # one-CDP apertures: every pick is a tie
+
+
+@pytest.mark.parametrize("nb,tau,ns,apm", [(21, 1, 300, 50), (9, 2, 331, 75), (5, 0, 500, 25), (21, 1, 700, 5)])
+def test_certified_repick_gives_the_fp64_picks(nb, tau, ns, apm):
+    """The re-pick in pairs of FP32 numbers against the same plan's FP64 re-pick (plans that
+    keep the extra attributes take FP64 throughout): same picks, semblances and stacks, bit
+    for bit, with few and many traces per aperture (apm 5: one CDP, all A and B tie)."""
+    s = _survey(nb, tau, ns, apm, ncdp=9, fold=14, na=4)
+    g = oracle.gather(s.headers, s.samples, "crs", s.params["aph"], s.params["apm"], real=np.float64)
+    out = []
+    for attrs in (0, 1):
+        for repick in (semb.REPICK_NEAR_TIES, semb.REPICK_ALWAYS):
+            with semb.Plan(semb.params(semb.CRS, mode=semb.BATCHED, attrs=attrs, repick=repick, **s.params)) as p:
+                p.upload(_arrays(g).view())
+                p.run()
+                out.append(p.download())
+                assert p.stats()["repicked"] > 0
+    for a, b in ((out[0], out[2]), (out[1], out[3])):
+        for x, y in zip(a, b):
+            assert np.array_equal(x, y)
