@@ -51,7 +51,7 @@ constexpr int kGridNeighbours = 2048;
 constexpr int kMinStage = 512;
 int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, float c, float* out, cudaStream_t st);
 int launch_repick(int w, RepickParams R, int sms, cudaStream_t st);
-int launch_crs_de(int w, const DeParams& R, cudaStream_t st);
+int launch_crs_de(int w, const DeParams& R, KParams P, cudaStream_t st);
 bool filter_exists(int form, int w, int brun, int pipe, int lay);
 int filter_shape(int w, int nb, int* rc, int* nt);
 size_t filter_smem(int form, int storage, int nt, int cap);
@@ -166,6 +166,7 @@ struct semb_plan {
   std::vector<int32_t> aperture;   // aperture traces per CDP (host copy)
   // CRS-DE (ngen > 0): the single-precision grid and the picked parameters
   float* d_grid = nullptr;
+  float* d_de_box = nullptr;   // the search box as pass bounds
   float* d_de_a = nullptr;
   float* d_de_b = nullptr;
   float* d_de_c = nullptr;
@@ -316,6 +317,7 @@ void free_data(semb_plan* pl, bool keep_reusable = false) {
   release(pl->d_idx2);
   release(pl->d_err64);
   release(pl->d_grid);
+  release(pl->d_de_box);
   release(pl->d_de_a);
   release(pl->d_de_b);
   release(pl->d_de_c);
@@ -1214,6 +1216,15 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
     SEMB_TRY(dev_alloc(&pl->d_grid, grid.size()));
     SEMB_CUDA(cudaMemcpyAsync(pl->d_grid, grid.data(), grid.size() * 4, cudaMemcpyHostToDevice, st));
     SEMB_CUDA(cudaStreamSynchronize(st));
+    const float lo[3] = {(float)p.a0, (float)p.b0, (float)(p.c0 * kFactor)};
+    const float hi[3] = {(float)p.a1, (float)p.b1, (float)(p.c1 * kFactor)};
+    float box[8] = {};
+    for (int d = 0; d < 3; ++d) {
+      box[2 * d] = std::min(lo[d], hi[d]);
+      box[2 * d + 1] = std::max(lo[d], hi[d]);
+    }
+    SEMB_TRY(dev_alloc(&pl->d_de_box, 8));
+    SEMB_CUDA(cudaMemcpy(pl->d_de_box, box, sizeof(box), cudaMemcpyHostToDevice));
     SEMB_TRY(dev_alloc(&pl->d_de_a, nout));
     SEMB_TRY(dev_alloc(&pl->d_de_b, nout));
     SEMB_TRY(dev_alloc(&pl->d_de_c, nout));
@@ -1400,7 +1411,8 @@ int enqueue_run(semb_plan* pl, bool timed) {
     D.stk = pl->d_stk;
     SEMB_CUDA(cudaMemsetAsync(pl->d_ctr, 0xff, (size_t)pl->ncdps * pl->ns * 4, st));
     if (timed) SEMB_CUDA(cudaEventRecord(pl->ev[1], st));
-    SEMB_TRY(launch_crs_de(pl->w, D, st));
+    P.pass_bounds = pl->d_de_box;
+    SEMB_TRY(launch_crs_de(pl->w, D, P, st));
     ++launches;
     if (timed) {
       SEMB_CUDA(cudaEventRecord(pl->ev[2], st));
