@@ -38,13 +38,13 @@ int search_variant(int method, int form, int w, int v, int* rc, int* minb, int* 
 // Candidate slots of one (A, C) group's run of nb B values padded to a multiple of rc.
 static int brun_slots(int nb, int rc) { return (std::max(nb, 1) + rc - 1) / rc * rc; }
 
-// Launch shape of semb_plain_kernel for ncand candidates at rc per thread and at most
+// Launch shape of semb_plain_kernel and semb_ring_kernel for ncand candidates at rc per thread and at most
 // max_warps warps per SM: warps per CTA and CTAs per SM (several where one needs few
 // warps).  Returns its cost, time per aperture trace in candidates per lane: a pass of nw
 // warps takes its schedulers ceil(nw / 4) warps' time each, and not less than `few` warps'
 // (with fewer, the latency of a warp's own chain shows).
 double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas) {
-  const double few = rc == 8 ? 2.5 : 4.0;
+  const double few = rc == 4 ? 4.0 : 2.5;
   double best = 1e300;
   for (int nw = max_warps; nw >= 4; --nw) {
     const int npass = (ncand + nw * rc - 1) / (nw * rc), k = std::min(4, max_warps / nw);
@@ -68,19 +68,41 @@ static int plain_variant(int ncand) {
   return plain_shape(ncand, 4, 26, &nw, &k) < 0.97 * plain_shape(ncand, 8, 16, &nw, &k) ? 1 : 0;
 }
 
+// Batched CMP: the ring kernel (30, 31) or -1 for the two-barrier one, which runs two CTAs
+// per SM whatever the candidate count.  `fold`: the aperture traces of the average
+// trace-evaluation.  Where one ring CTA has to fill an SM its planner, merges and staging
+// show on small folds: it pays from about 60 traces (150 for w = 3), and always where
+// several CTAs share the SM.  Measured, ring / two-barrier (ms): w = 5, 256 candidates, fold
+// 12 to 240 (mean 126) 9.34 / 10.29, fold 60 3.41 / 3.46, fold 12 1.20 / 1.01; w = 3, 101
+// candidates, fold 200 1.93 / 2.05, fold 60 1.38 / 1.36; 40 candidates, fold 60 0.58 / 0.68,
+// fold 12 0.33 / 0.38; w = 11, 90 candidates, fold 37 0.46 / 0.57; w = 15, 200 candidates 1.21
+// / 1.95; w = 7, 64 candidates 0.32 / 0.27.
+static int ring_variant(int w, int ncand, double fold) {
+  int nw = 0, k8 = 1, k10 = 1;
+  if (w >= 7) return ncand >= 80 && fold >= 30.0 ? 31 : -1;
+  const double c8 = plain_shape(ncand, 8, 16, &nw, &k8), c10 = plain_shape(ncand, 10, 12, &nw, &k10);
+  const int v = c10 < c8 ? 31 : 30;
+  if ((v == 31 ? k10 : k8) >= 2) return v;
+  return fold >= (w == 3 ? 150.0 : 60.0) ? v : -1;
+}
+
 // Variant a plan starts with (before any autotuning), the fastest measured on GB300
 // for the benchmark workloads of each window: for CRS the pipelined B-run kernel
 // (packed value/difference staging with a two-way trace unroll and the central traces'
-// sums shared over A and B for w = 3, packed pairs otherwise); for CMP the
-// two-barrier kernel with packed pairs (w = 3) or packed pairs formed by scalar FMAs
-// (w = 5); variant 0 elsewhere.  For CRS with w = 3 the B-run length follows the
+// sums shared over A and B for w = 3, packed pairs otherwise); for CMP the ring kernel
+// where ring_variant() says (fold > 0), else the two-barrier kernel with packed pairs (w =
+// 3) or packed pairs formed by scalar FMAs (w = 5); variant 0 elsewhere.  For CRS with w = 3 the B-run length follows the
 // grid's nb: runs of 7 (variant 30, 512 threads) unless nb pads less to a multiple of
 // 8 (variant 33, 384 threads; nb = 31 takes 32 slots per (A, C) instead of 35; per
 // slot the two run at the same speed).  fallback_variant() is the one to use where the
 // default does not fit the plan (a grid whose passes span more C values than the
 // central-trace sharing takes).
-int default_variant(int method, int form, int w, int nb, int ncand) {
+int default_variant(int method, int form, int w, int nb, int ncand, double fold) {
   if (form != FORM_FAST) return w <= 5 ? plain_variant(ncand) : 0;
+  if (method == METHOD_CMP && fold > 0.0) {
+    const int v = ring_variant(w, ncand, fold);
+    if (v >= 0) return v;
+  }
   if (method == METHOD_CRS && w == 3) return brun_slots(nb, 8) < brun_slots(nb, 7) ? 33 : 30;
   if (method == METHOD_CRS && w <= 5) return 14;
   if (method == METHOD_CMP && w == 3) return 8;

@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(NT, 1) semb_plain_kernel(KParams P) {
     const uint32_t plane = smem_u32(plane_at(c));
     const uint32_t top = plane + 4u * (uint32_t)P.cap;
     const float2 T2 = make_float2(Tsec, Tsec);
+#pragma unroll 2
     for (int e = 0; e < n; ++e) {
       const float4 g = meta->geo[e];
       const float2 gx = make_float2(g.x, g.x), gy = make_float2(g.y, g.y), gz = make_float2(g.z, g.z);

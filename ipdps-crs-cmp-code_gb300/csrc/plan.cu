@@ -23,6 +23,7 @@
 #include "plain_kernel.cuh"
 #include "plan_kernels.cuh"
 #include "refine_kernel.cuh"
+#include "ring_kernel.cuh"
 #include "semb_kernels.cuh"
 
 namespace semb {
@@ -40,7 +41,7 @@ constexpr int kBucketSplits = 3;
 constexpr int kBucketAp[kBucketSplits] = {1024, 384, 128};
 static_assert(kBucketSplits + 1 <= kMaxBuckets, "bucket table");
 int search_occupancy(int method, int form, int w, int variant, int nwarps, size_t smem, int* ctas_per_sm);
-int default_variant(int method, int form, int w, int nb, int ncand);
+int default_variant(int method, int form, int w, int nb, int ncand, double fold);
 double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas);
 int fallback_variant(int method, int form, int w, int nb);
 int grid_neighbours(int ncdps, const float* d_fmx, const float* d_fmy, int apm, int64_t* d_off, int32_t** d_list,
@@ -590,7 +591,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
       best_nw = nw;
     }
   }
-  if (pipe == 3) plain_shape(nslots, rc, nt / 32, &best_nw, &minb);
+  if (pipe >= 3) plain_shape(nslots, rc, nt / 32, &best_nw, &minb);
   const int cpp = best_nw * rc;
   const int npass = (nslots + cpp - 1) / cpp;
   // Z0 variants: each pass's C indices (C is outermost in the search order, so they are
@@ -625,17 +626,18 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   // plan's stage_cap, which also bounds it from above).
   const bool small_stages = form == FORM_FAST && glob;
   const int store = (form == FORM_FAST) ? p.storage : SEMB_STORE_F32;
-  // the ring kernel's CTAs share the SM only where each still holds a whole trace's window
-  // in every plane
-  while (pipe == 3 && minb > 1 && plain_layout((int)pl->pitch + 16, nt).total > (227 * 1024) / (size_t)minb - 1024) --minb;
-  const size_t budget = (227 * 1024) / minb - 1024;
-  int cap = form == FORM_PLAIN ? 32768 : 8192;
-  if (form == FORM_FAST && pl->stage_cap > 0) cap = std::min(cap, pl->stage_cap);
   auto smem_of = [&](int cp) {
-    return pipe == 3 ? plain_layout(cp, nt).total
-           : pipe    ? pipe_layout(rc, cp, store, nt, lay, z0).total
-                     : smem_layout(form, rc, cp, store, nt, lay).total;
+    return pipe == 4   ? ring_layout(rc, cp, store, nt).total
+           : pipe == 3 ? plain_layout(cp, nt).total
+           : pipe      ? pipe_layout(rc, cp, store, nt, lay, z0).total
+                       : smem_layout(form, rc, cp, store, nt, lay).total;
   };
+  // the ring kernels' CTAs share the SM only where each still holds a whole trace's window
+  // in every plane
+  while (pipe >= 3 && minb > 1 && smem_of((int)pl->pitch + 16) > (227 * 1024) / (size_t)minb - 1024) --minb;
+  const size_t budget = (227 * 1024) / minb - 1024;
+  int cap = form == FORM_PLAIN || pipe == 4 ? 32768 : 8192;
+  if (form == FORM_FAST && pl->stage_cap > 0) cap = std::min(cap, pl->stage_cap);
   if (lay == LAY_X3) cap = std::min(cap, kXPlane - kZeroSlots);
   while (cap > 64 && smem_of(cap) > budget) cap -= 64;
   int min_cap = (int)pl->pitch + 16;
@@ -1232,8 +1234,13 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   pl->aperture.resize(g->ncdps);
   for (int i = 0; i < g->ncdps; ++i) pl->aperture[i] = (int32_t)(ap_off[i + 1] - ap_off[i]);
 
-  // the default variant of this method and window; variant 0 where it does not fit
-  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand)) != SEMB_OK &&
+  // the default variant of this method and window, given the aperture of the average
+  // trace-evaluation; where it does not fit this plan's traces the next best, then variant 0
+  double ap2 = 0.0;
+  for (int i = 0; i < g->ncdps; ++i) ap2 += (double)pl->aperture[i] * pl->aperture[i];
+  const double fold = ap2 / (double)std::max<int64_t>(pl->nap, 1);
+  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, fold)) != SEMB_OK &&
+      set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, 0.0)) != SEMB_OK &&
       set_all(pl, fallback_variant(p.method, form, pl->w, p.nb)) != SEMB_OK)
     SEMB_TRY(set_all(pl, 0));
   // streamed: the other chunks' copies, after the set-up's own small copies

@@ -22,6 +22,7 @@
 #include "common.h"
 #include "pipe_kernel.cuh"
 #include "plain_kernel.cuh"
+#include "ring_kernel.cuh"
 #include "semb_kernels.cuh"
 
 namespace semb {
@@ -32,7 +33,8 @@ struct SearchEntry {
   int minb;
   int brun;   // candidates laid out as B runs of RC (CRS)
   int nt;     // threads per CTA
-  int pipe;   // 1: semb_pipe_kernel (decoupled staging ring), 3: semb_plain_kernel, 0: semb_search_kernel
+  int pipe;   // 1: semb_pipe_kernel (decoupled staging ring), 3: semb_plain_kernel, 4: semb_ring_kernel,
+              // 0: semb_search_kernel
   int lay;    // staging layout (LAY_*)
   int glob;   // 1: stages may be smaller than a trace (long windows read global memory)
   int z0;     // 1: the central traces' sums are shared over A and B (semb_pipe_kernel Z0)
@@ -58,6 +60,18 @@ template <int METHOD, int W, int RC, int MINB, int LAY = LAY_P2, bool BRUN = fal
 SearchEntry pipe_entry() {
   return {(const void*)semb_pipe_kernel<METHOD, W, RC, MINB, LAY, BRUN, NT, TU, GLOB, Z0>, RC, MINB, BRUN ? 1 : 0, NT, 1,
           LAY, GLOB ? 1 : 0, Z0 ? 1 : 0};
+}
+
+// CMP, batched: item pairs in the staging ring (variant 30: 8 candidates per thread in up to
+// 16 warps, 4 from w = 7 on; 31: 10 and 6 in up to 12 warps)
+template <int METHOD, int W>
+SearchEntry ring_entry(int variant) {
+  if constexpr (METHOD == METHOD_CMP) {
+    constexpr int R0 = W <= 5 ? 8 : 4, R1 = W <= 5 ? 10 : 6;
+    if (variant == 30) return {(const void*)semb_ring_kernel<W, R0, 512>, R0, 1, 0, 512, 4, LAY_QUAD, 0, 0};
+    if (variant == 31) return {(const void*)semb_ring_kernel<W, R1, 384>, R1, 1, 0, 384, 4, LAY_QUAD, 0, 0};
+  }
+  return {nullptr, 0, 0, 0, 0, 0, 0, 0, 0};
 }
 
 // Plain form: windows up to 5 in the ring kernel, with 8 candidates per thread in up to 16
@@ -98,6 +112,7 @@ SearchEntry search_entry(int w, int variant) {
   // fast form
   switch (w) {
     case 1:
+      if (METHOD == METHOD_CMP && (variant == 30 || variant == 31)) return ring_entry<METHOD, 1>(variant);
       if (variant == 0) return entry<METHOD, FORM, 1, 8, 2>();
       if (variant == 1) return entry<METHOD, FORM, 1, 4, 3>();
       if (METHOD == METHOD_CRS && variant == 4) return entry<METHOD, FORM, 1, 7, 2, LAY_QUAD, true>();
@@ -108,6 +123,7 @@ SearchEntry search_entry(int w, int variant) {
       if (METHOD == METHOD_CRS && variant == 14) return pipe_entry<METHOD, 1, 7, 1, LAY_QUAD, true, 512>();
       break;
     case 3:
+      if (METHOD == METHOD_CMP && (variant == 30 || variant == 31)) return ring_entry<METHOD, 3>(variant);
       if (variant == 0) return entry<METHOD, FORM, 3, (METHOD == METHOD_CMP ? 8 : 6), 2>();
       if (variant == 1) return entry<METHOD, FORM, 3, 4, 3>();
       if (variant == 2) return entry<METHOD, FORM, 3, (METHOD == METHOD_CMP ? 6 : 8), 2>();
@@ -159,6 +175,7 @@ SearchEntry search_entry(int w, int variant) {
       }
       break;
     case 5:
+      if (METHOD == METHOD_CMP && (variant == 30 || variant == 31)) return ring_entry<METHOD, 5>(variant);
       if (variant == 0) return entry<METHOD, FORM, 5, (METHOD == METHOD_CMP ? 8 : 6), 2>();
       if (variant == 1) return entry<METHOD, FORM, 5, 4, 3>();
       if (variant == 2) return entry<METHOD, FORM, 5, (METHOD == METHOD_CMP ? 6 : 4), 2>();
@@ -190,11 +207,11 @@ SearchEntry search_entry(int w, int variant) {
       if (variant == 26) return xp_entry<METHOD, FORM, 5, (METHOD == METHOD_CMP ? 8 : 6), 2, LAY_PD5S>();
       break;
 #if SEMB_WIDE_WINDOWS
-    case 7: if (variant == 0) return entry<METHOD, FORM, 7, 4, 2>(); break;
-    case 9: if (variant == 0) return entry<METHOD, FORM, 9, 4, 2>(); break;
-    case 11: if (variant == 0) return entry<METHOD, FORM, 11, 3, 2>(); break;
-    case 13: if (variant == 0) return entry<METHOD, FORM, 13, 3, 2>(); break;
-    case 15: if (variant == 0) return entry<METHOD, FORM, 15, 2, 2>(); break;
+    case 7: if (variant == 0) return entry<METHOD, FORM, 7, 4, 2>(); return ring_entry<METHOD, 7>(variant);
+    case 9: if (variant == 0) return entry<METHOD, FORM, 9, 4, 2>(); return ring_entry<METHOD, 9>(variant);
+    case 11: if (variant == 0) return entry<METHOD, FORM, 11, 3, 2>(); return ring_entry<METHOD, 11>(variant);
+    case 13: if (variant == 0) return entry<METHOD, FORM, 13, 3, 2>(); return ring_entry<METHOD, 13>(variant);
+    case 15: if (variant == 0) return entry<METHOD, FORM, 15, 2, 2>(); return ring_entry<METHOD, 15>(variant);
 #endif
     default: break;
   }
