@@ -38,11 +38,11 @@ int search_variant(int method, int form, int w, int v, int* rc, int* minb, int* 
 // Candidate slots of one (A, C) group's run of nb B values padded to a multiple of rc.
 static int brun_slots(int nb, int rc) { return (std::max(nb, 1) + rc - 1) / rc * rc; }
 
-// Launch shape of semb_plain_kernel and semb_ring_kernel for ncand candidates at rc per thread and at most
-// max_warps warps per SM: warps per CTA and CTAs per SM (several where one needs few
-// warps).  Returns its cost, time per aperture trace in candidates per lane: a pass of nw
-// warps takes its schedulers ceil(nw / 4) warps' time each, and not less than `few` warps'
-// (with fewer, the latency of a warp's own chain shows).
+// Launch shape of semb_plain_kernel and semb_ring_kernel for ncand candidates at rc per
+// thread and at most max_warps warps per SM: warps per CTA and CTAs per SM (several where
+// one needs few warps).  Returns its cost, time per aperture trace in candidates per lane:
+// a pass of nw warps takes its schedulers ceil(nw / 4) warps' time each, and not less than
+// `few` warps' (with fewer, the latency of a warp's own chain shows).
 double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas) {
   const double few = rc == 4 ? 4.0 : 2.5;
   double best = 1e300;
@@ -59,31 +59,50 @@ double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas) {
 }
 
 // Plain form, windows up to 5: 8 candidates per thread (variant 0) unless 4 (variant 1)
-// use the warps better.  Measured, variant 0 / 1 / the two-barrier kernel (ms): 256
-// candidates, w = 5: 8.66 / 9.21 / 11.44; 200, w = 3: 3.24 / 3.19 / 5.03; 101, w = 3: 1.86 /
-// 1.74 / 2.37; 90, w = 5: 1.98 / 2.09 / 2.57; 64, w = 3: 1.96 / 2.19 / 2.42; 33, w = 1: 0.50 /
-// 0.44 / 0.80.
-static int plain_variant(int ncand) {
-  int nw, k;
-  return plain_shape(ncand, 4, 26, &nw, &k) < 0.97 * plain_shape(ncand, 8, 16, &nw, &k) ? 1 : 0;
+// use the warps better; where both come out even and 8 need one pass of a whole SM, 4 for
+// the windows whose per-candidate chain is short.  Measured, variant 0 / 1 / the two-barrier
+// kernel (ms): 256 candidates, w = 5: 8.66 / 9.21 / 11.44; 200, w = 3: 3.24 / 3.19 / 5.03;
+// 101, w = 3: 1.86 / 1.74 / 2.37; 90, w = 5: 1.98 / 2.09 / 2.57; 64, w = 3: 1.96 / 2.19 /
+// 2.42; 33, w = 1: 0.50 / 0.44 / 0.80; 125, w = 1, 234 tasks: 0.100 / 0.083 / 0.096, w = 3:
+// 0.125 / 0.114 / 0.131, w = 5: 0.156 / 0.159 / 0.163.
+static int plain_variant(int w, int ncand) {
+  int nw, k4, k8;
+  const double c4 = plain_shape(ncand, 4, 26, &nw, &k4), c8 = plain_shape(ncand, 8, 16, &nw, &k8);
+  return c4 < (w <= 3 && k8 == 1 && ncand <= 8 * nw ? 1.03 : 0.97) * c8 ? 1 : 0;
 }
 
-// Batched CMP: the ring kernel (30, 31) or -1 for the two-barrier one, which runs two CTAs
-// per SM whatever the candidate count.  `fold`: the aperture traces of the average
-// trace-evaluation.  Where one ring CTA has to fill an SM its planner, merges and staging
-// show on small folds: it pays from about 60 traces (150 for w = 3), and always where
-// several CTAs share the SM.  Measured, ring / two-barrier (ms): w = 5, 256 candidates, fold
-// 12 to 240 (mean 126) 9.34 / 10.29, fold 60 3.41 / 3.46, fold 12 1.20 / 1.01; w = 3, 101
-// candidates, fold 200 1.93 / 2.05, fold 60 1.38 / 1.36; 40 candidates, fold 60 0.58 / 0.68,
-// fold 12 0.33 / 0.38; w = 11, 90 candidates, fold 37 0.46 / 0.57; w = 15, 200 candidates 1.21
-// / 1.95; w = 7, 64 candidates 0.32 / 0.27.
-static int ring_variant(int w, int ncand, double fold) {
-  int nw = 0, k8 = 1, k10 = 1;
-  if (w >= 7) return ncand >= 80 && fold >= 30.0 ? 31 : -1;
-  const double c8 = plain_shape(ncand, 8, 16, &nw, &k8), c10 = plain_shape(ncand, 10, 12, &nw, &k10);
-  const int v = c10 < c8 ? 31 : 30;
-  if ((v == 31 ? k10 : k8) >= 2) return v;
-  return fold >= (w == 3 ? 150.0 : 60.0) ? v : -1;
+// Batched CMP: the ring kernel (30, 31) or -1 for the two-barrier one.  `fold`: the aperture
+// traces of the average trace-evaluation; `tasks_per_sm` of the plan.
+//
+// Up to w = 5 the two-barrier kernel evaluates 64 candidates per pass on two CTAs per SM.
+// The ring kernel is ahead where its shape computes at most 0.85 of the padded candidates
+// (20 to 40, 65 to 95, 129 to 160 of them, ...); where both compute the same, its planner,
+// staging and merges show on small folds: from 110 traces it pays with several passes a
+// chunk, from 150 with w = 1.  Measured, ring / two-barrier, folds of 30, 62 and 150: w = 5,
+// 160 candidates 0.83, 0.82, 0.81; 80 0.86, 0.81, 0.80; 256 1.11, 1.03, 0.95 (uneven folds of
+// 12 to 240 9.34 / 10.29 ms); 128 1.27, 1.12, 0.98; w = 3, 33 candidates 0.98, 0.88, 0.87; 64
+// 1.01, 0.99, 1.00; w = 1, 128 1.27, 1.06, 0.86.
+//
+// From w = 7 on the two-barrier kernel's entries of 16 bytes per window sample and its few
+// candidates per thread put it behind from 80 candidates on, unless those fill its warps on
+// small folds (w = 7, 128 candidates, fold 20: 1.17; 40: 1.06; 90: 0.96) or, at w = 15, by
+// its narrow passes (80 candidates 1.00).  Several ring CTAs to the SM need the tasks to
+// fill them.  Measured: w = 7, 80 candidates 0.77; w = 11, 90 0.46 / 0.57 ms, 128 0.72, 200
+// 0.70; w = 15, 101 0.66, 200 0.63, 256 0.88.
+static int ring_variant(int w, int ncand, double fold, double tasks_per_sm) {
+  int nw = 0, k0 = 1, k1 = 1;
+  if (w >= 7) {
+    const double c4 = plain_shape(ncand, 4, 16, &nw, &k0), c6 = plain_shape(ncand, 6, 12, &nw, &k1);
+    const int v = c6 <= 1.03 * c4 ? 31 : 30;
+    if (ncand < (w >= 13 ? 96 : 80) || ((v == 31 ? k1 : k0) > 1 && tasks_per_sm < 3.0)) return -1;
+    return w <= 9 && ncand % 32 == 0 && fold < 60.0 ? -1 : v;
+  }
+  const double c8 = plain_shape(ncand, 8, 16, &nw, &k0), c10 = plain_shape(ncand, 10, 12, &nw, &k1);
+  const int v = c10 <= c8 ? 31 : 30;
+  const double pad = (ncand + 63) / 64 * 16.0, c = std::min(c8, c10);
+  if (c <= 0.85 * pad) return v;
+  if (fold >= 110.0 && ncand > 128 && c8 <= pad) return 30;
+  return w == 1 && fold >= 150.0 && c <= pad ? v : -1;
 }
 
 // Variant a plan starts with (before any autotuning), the fastest measured on GB300
@@ -91,16 +110,16 @@ static int ring_variant(int w, int ncand, double fold) {
 // (packed value/difference staging with a two-way trace unroll and the central traces'
 // sums shared over A and B for w = 3, packed pairs otherwise); for CMP the ring kernel
 // where ring_variant() says (fold > 0), else the two-barrier kernel with packed pairs (w =
-// 3) or packed pairs formed by scalar FMAs (w = 5); variant 0 elsewhere.  For CRS with w = 3 the B-run length follows the
-// grid's nb: runs of 7 (variant 30, 512 threads) unless nb pads less to a multiple of
-// 8 (variant 33, 384 threads; nb = 31 takes 32 slots per (A, C) instead of 35; per
-// slot the two run at the same speed).  fallback_variant() is the one to use where the
-// default does not fit the plan (a grid whose passes span more C values than the
-// central-trace sharing takes).
-int default_variant(int method, int form, int w, int nb, int ncand, double fold) {
-  if (form != FORM_FAST) return w <= 5 ? plain_variant(ncand) : 0;
+// 3) or packed pairs formed by scalar FMAs (w = 5); variant 0 elsewhere.  For CRS with w = 3
+// the B-run length follows the grid's nb: runs of 7 (variant 30, 512 threads) unless nb
+// pads less to a multiple of 8 (variant 33, 384 threads; nb = 31 takes 32 slots per (A, C)
+// instead of 35; per slot the two run at the same speed).  fallback_variant() is the one to
+// use where the default does not fit the plan (a grid whose passes span more C values than
+// the central-trace sharing takes).
+int default_variant(int method, int form, int w, int nb, int ncand, double fold, double tasks_per_sm) {
+  if (form != FORM_FAST) return w <= 5 ? plain_variant(w, ncand) : 0;
   if (method == METHOD_CMP && fold > 0.0) {
-    const int v = ring_variant(w, ncand, fold);
+    const int v = ring_variant(w, ncand, fold, tasks_per_sm);
     if (v >= 0) return v;
   }
   if (method == METHOD_CRS && w == 3) return brun_slots(nb, 8) < brun_slots(nb, 7) ? 33 : 30;
