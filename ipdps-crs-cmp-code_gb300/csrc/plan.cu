@@ -263,17 +263,41 @@ void drop_graph(semb_plan* pl) {
   pl->chunks_dirty = true;
 }
 
-// Device buffer *p of n elements, kept from the previous upload when it is large
-// enough (re-uploads of a survey of the same size then allocate nothing).
 template <typename T>
-int dev_reuse(semb_plan* pl, T** p, size_t n) {
+void dev_release(semb_plan* pl, T*& p) {
+  pl->caps.erase(&p);
+  dev_free(p);
+}
+
+// Gives back the buffers that a plan can do without (the re-pick's paired geometry and the
+// filter's lists); false where there are none.
+bool drop_optional(semb_plan* pl) {
+  const bool any = pl->d_ap_ff || pl->d_head || pl->d_pool || pl->d_fb_tasks;
+  dev_release(pl, pl->d_ap_ff);
+  dev_release(pl, pl->d_head);
+  dev_release(pl, pl->d_pool);
+  dev_release(pl, pl->d_fb_tasks);
+  return any;
+}
+
+// Device buffer *p of n elements, kept from the previous upload when it is large
+// enough (re-uploads of a survey of the same size then allocate nothing).  An upload that
+// runs out of memory gives the optional buffers back before it fails (no launch
+// configuration holds them then).
+template <typename T>
+int dev_reuse(semb_plan* pl, T** p, size_t n, bool optional = false) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
   auto it = pl->caps.find(p);
   if (*p && it != pl->caps.end() && it->second >= bytes) return SEMB_OK;
   if (*p) cudaFree(*p);
   *p = nullptr;
   pl->caps.erase(p);
-  SEMB_TRY(dev_alloc(p, n));
+  int rc = dev_alloc(p, n);
+  if (rc == SEMB_E_NOMEM) {
+    cudaGetLastError();
+    if (!optional && !pl->uploaded && drop_optional(pl)) rc = dev_alloc(p, n);
+  }
+  if (rc != SEMB_OK) return rc;
   pl->caps[p] = bytes;
   return SEMB_OK;
 }
@@ -518,9 +542,16 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   // the lists and tables; without the memory for them the search is direct
   const size_t nout = (size_t)pl->ncdps * pl->ns;
   pl->pool_cap = (int)std::min<size_t>(nout * kFilterPool + 4096, INT32_MAX);
-  if (dev_reuse(pl, &pl->d_head, nout) != SEMB_OK || dev_reuse(pl, &pl->d_pool, (size_t)pl->pool_cap) != SEMB_OK ||
-      dev_reuse(pl, &pl->d_fb_tasks, pl->ntasks) != SEMB_OK || dev_reuse(pl, &pl->d_fb_count, 6) != SEMB_OK ||
-      dev_alloc(&f.d_cand, npad) != SEMB_OK || dev_alloc(&f.d_pass_bounds, bounds.size()) != SEMB_OK) {
+  if (dev_reuse(pl, &pl->d_head, nout, true) != SEMB_OK ||
+      dev_reuse(pl, &pl->d_pool, (size_t)pl->pool_cap, true) != SEMB_OK ||
+      dev_reuse(pl, &pl->d_fb_tasks, pl->ntasks, true) != SEMB_OK) {
+    dev_release(pl, pl->d_head);   // another configuration's filter would have found them
+    dev_release(pl, pl->d_pool);
+    dev_release(pl, pl->d_fb_tasks);
+    return SEMB_OK;
+  }
+  if (dev_reuse(pl, &pl->d_fb_count, 6, true) != SEMB_OK || dev_alloc(&f.d_cand, npad) != SEMB_OK ||
+      dev_alloc(&f.d_pass_bounds, bounds.size()) != SEMB_OK) {
     cudaGetLastError();
     dev_free(f.d_cand);
     dev_free(f.d_pass_bounds);
@@ -1054,7 +1085,7 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   // the re-pick's geometry in pairs of floats (the extra attributes take the FP64 values);
   // without the memory for it the re-pick is FP64 throughout
   const bool ff = p.method == SEMB_CRS && p.mode == SEMB_BATCHED && p.repick != SEMB_REPICK_OFF && !p.attrs &&
-                  dev_reuse(pl, &pl->d_ap_ff, 2 * (size_t)pl->nap) == SEMB_OK;
+                  dev_reuse(pl, &pl->d_ap_ff, 2 * (size_t)pl->nap, true) == SEMB_OK;
   if (!ff) cudaGetLastError();
   // azimuth direction for the signed midpoint displacement (SEMB_DM_SIGNED)
   const double az = p.azimuth * 3.14159265358979323846 / 180.0;
