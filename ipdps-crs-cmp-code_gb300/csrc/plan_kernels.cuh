@@ -675,9 +675,12 @@ __device__ void repick_item(const RepickParams& R, const int64_t item, const int
 // Final pick per (CDP, t0), R.per_warp consecutive items per warp: each lane screens one
 // item (no candidate above 0, or no near tie: the FP32 pick stands and the lane writes
 // it), then the warp takes the near-tie items one after the other (repick_item), all
-// lanes on one item's FP64 evaluation.
+// lanes on one item's evaluation.  Two CTAs per SM, 128 registers: with 64 the wide windows'
+// sums spill, with 255 one CTA does not cover its latency (100 CMPs x 1000, fold 30, 64
+// velocities: w = 5 56 us at 64 registers, 44 so; w = 9 109, 95, and 122 at 255; w = 11 126,
+// 106, 125; 200 CMPs of fold 8, w = 15 253, 181, 250).
 template <int W>
-static __global__ void __launch_bounds__(256, W <= 5 ? 2 : 1) k_repick(RepickParams R) {
+static __global__ void __launch_bounds__(256, 2) k_repick(RepickParams R) {
   const int lane = threadIdx.x & 31;
   const int64_t base = R.item0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * R.per_warp;
   if (base >= R.item_end) return;
