@@ -169,13 +169,14 @@ int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, 
 // fewer where that would leave the GPU's warps without work, as the near ties of a warp's
 // items run one after the other: 64 warps' worth of items per SM for CRS, most of whose items
 // are near ties (24 CDPs x 601 samples, w = 5: 3.2 ms at 32 per warp in FP64; 0.23 so, in
-// pairs of FP32 numbers), 8 for CMP, where 1% are and the screening of the others counts (75 x
-// 751, w = 11: 2% of the whole pass).
+// pairs of FP32 numbers).  For CMP 1% are, and the screening of the others counts up to w = 5
+// (100 x 1000, w = 5: 44 us at 8 warps' worth, 54 at 32); a wider window's ties are the longer
+// ones (75 x 751, w = 11: 147 us at 8, 114 at 16, 109 at 32; 100 x 1000, w = 15: 183, 183, 136).
 int launch_repick(int w, RepickParams R, int sms, cudaStream_t st) {
   const int64_t items = R.item_end - R.item0;
   if (items <= 0) return SEMB_OK;
   R.per_warp = 32;
-  while (R.per_warp > 1 && items < (int64_t)sms * (R.method == METHOD_CRS ? 64 : 8) * R.per_warp) R.per_warp /= 2;
+  while (R.per_warp > 1 && items < (int64_t)sms * (R.method == METHOD_CRS ? 64 : w <= 5 ? 8 : 32) * R.per_warp) R.per_warp /= 2;
   const int grid = (int)((items + 8 * R.per_warp - 1) / (8 * R.per_warp));   // 8 warps per CTA
   switch (w) {
     case 1: k_repick<1><<<grid, 256, 0, st>>>(R); break;
