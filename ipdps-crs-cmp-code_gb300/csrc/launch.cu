@@ -89,8 +89,16 @@ static int plain_variant(int w, int ncand) {
 // its narrow passes (80 candidates 1.00).  Several ring CTAs to the SM need the tasks to
 // fill them.  Measured: w = 7, 80 candidates 0.77; w = 11, 90 0.46 / 0.57 ms, 128 0.72, 200
 // 0.70; w = 15, 101 0.66, 200 0.63, 256 0.88.
-static int ring_variant(int w, int ncand, double fold, double tasks_per_sm) {
+//
+// Records whose last tile of 32 samples reaches more than 3% beyond the end: its items
+// take the range-checked path, which costs 31 more than a third (w = 5, 34 candidates, 304
+// samples: 31 1.20, 30 1.03, 80 candidates 1.09 and 0.98; 320 samples: 0.90 and 0.92).
+static int ring_variant(int w, int ncand, int ns, double fold, double tasks_per_sm) {
   int nw = 0, k0 = 1, k1 = 1;
+  if (((ns + 31) / 32 * 32 - ns) * 100 > 3 * ns) {
+    if (w > 5 || (w > 1 && ncand > 24 && ncand <= 64)) return -1;
+    return plain_shape(ncand, 8, 16, &nw, &k0) <= 0.85 * ((ncand + 63) / 64 * 16.0) ? 30 : -1;
+  }
   if (w >= 7) {
     const double c4 = plain_shape(ncand, 4, 16, &nw, &k0), c6 = plain_shape(ncand, 6, 12, &nw, &k1);
     const int v = c6 <= 1.03 * c4 ? 31 : 30;
@@ -116,10 +124,10 @@ static int ring_variant(int w, int ncand, double fold, double tasks_per_sm) {
 // instead of 35; per slot the two run at the same speed).  fallback_variant() is the one to
 // use where the default does not fit the plan (a grid whose passes span more C values than
 // the central-trace sharing takes).
-int default_variant(int method, int form, int w, int nb, int ncand, double fold, double tasks_per_sm) {
+int default_variant(int method, int form, int w, int nb, int ncand, int ns, double fold, double tasks_per_sm) {
   if (form != FORM_FAST) return w <= 5 ? plain_variant(w, ncand) : 0;
   if (method == METHOD_CMP && fold > 0.0) {
-    const int v = ring_variant(w, ncand, fold, tasks_per_sm);
+    const int v = ring_variant(w, ncand, ns, fold, tasks_per_sm);
     if (v >= 0) return v;
   }
   if (method == METHOD_CRS && w == 3) return brun_slots(nb, 8) < brun_slots(nb, 7) ? 33 : 30;

@@ -41,7 +41,7 @@ constexpr int kBucketSplits = 3;
 constexpr int kBucketAp[kBucketSplits] = {1024, 384, 128};
 static_assert(kBucketSplits + 1 <= kMaxBuckets, "bucket table");
 int search_occupancy(int method, int form, int w, int variant, int nwarps, size_t smem, int* ctas_per_sm);
-int default_variant(int method, int form, int w, int nb, int ncand, double fold, double tasks_per_sm);
+int default_variant(int method, int form, int w, int nb, int ncand, int ns, double fold, double tasks_per_sm);
 double plain_shape(int ncand, int rc, int max_warps, int* nwarps, int* ctas);
 int fallback_variant(int method, int form, int w, int nb);
 int grid_neighbours(int ncdps, const float* d_fmx, const float* d_fmy, int apm, int64_t* d_off, int32_t** d_list,
@@ -1270,8 +1270,8 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   double ap2 = 0.0;
   for (int i = 0; i < g->ncdps; ++i) ap2 += (double)pl->aperture[i] * pl->aperture[i];
   const double fold = ap2 / (double)std::max<int64_t>(pl->nap, 1), per_sm = (double)pl->ntasks / std::max(pl->sms, 1);
-  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, fold, per_sm)) != SEMB_OK &&
-      set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, 0.0, per_sm)) != SEMB_OK &&
+  if (set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, pl->ns, fold, per_sm)) != SEMB_OK &&
+      set_all(pl, default_variant(p.method, form, pl->w, p.nb, pl->ncand, pl->ns, 0.0, per_sm)) != SEMB_OK &&
       set_all(pl, fallback_variant(p.method, form, pl->w, p.nb)) != SEMB_OK)
     SEMB_TRY(set_all(pl, 0));
   // streamed: the other chunks' copies, after the set-up's own small copies
