@@ -66,10 +66,10 @@
 // second-order terms only where they count (moment_linear) gave 2%, the crossings above
 // and below the centre apart (half the slots each) 7%; two noted traces at a time was 10%
 // slower, and so was the main loop unrolled by four.
-// Measured on GB300, whole pass with the FP64 re-pick, direct kernels -> filter and refine:
-// 64 CDPs of the line (21 x 21 x 21, FP16) 172.3 -> 61.7 ms; 128 CDPs with apertures of 50
-// to 2000 traces 832 -> 281 ms; 48 such CDPs with 31 x 31 x 31 candidates (BF16) 621 -> 172
-// ms; plain form, 12 CDPs of the line 99.6 -> 9.3 ms.
+// Measured on GB300, whole pass with the re-pick, before this kernel and now: 64 CDPs of
+// the line (21 x 21 x 21, FP16) 172.5 -> 53.6 ms; 128 CDPs with apertures of 50 to 2000
+// traces 449 -> 151 ms; 48 such CDPs with 31 x 31 x 31 candidates (BF16) 690 -> 189 ms;
+// plain form, 12 CDPs of the line 99.6 -> 9.4 ms.
 #pragma once
 
 #include <type_traits>
