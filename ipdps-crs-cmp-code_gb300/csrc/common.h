@@ -22,6 +22,8 @@ static_assert((double)kEpsilonF < kEpsilon, "kEpsilonF must be the float just be
 constexpr double kFactor = 1e6;
 constexpr int kMaxWCmp = 16;
 constexpr int kMaxWCrs = 5;
+// Dynamic shared memory of one CTA, at most
+constexpr int kMaxDynamicSmem = 227 * 1024;
 
 }  // namespace semb
 

@@ -528,7 +528,7 @@ int launch_crs_de(int w, const DeParams& R, KParams P, cudaStream_t st) {
   if (cap < min_cap) cap = (min_cap + 63) & ~63;
   const size_t smem = de_layout(cap, R.np).total;
   void* args[] = {const_cast<DeParams*>(&R), &P};
-  if (smem > 227 * 1024) {
+  if (smem > kMaxDynamicSmem) {
     const void* lf = w == 1   ? (const void*)k_crs_de_long<1>
                      : w == 3 ? (const void*)k_crs_de_long<3>
                               : (const void*)k_crs_de_long<5>;
@@ -539,7 +539,7 @@ int launch_crs_de(int w, const DeParams& R, KParams P, cudaStream_t st) {
   P.cap = cap;
   const int grid = (int)((int64_t)R.ncdps * ((R.ns + kDeWarps - 1) / kDeWarps));
   // the most any plan takes: plans of other sizes share the kernel
-  SEMB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+  SEMB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem));
   SEMB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(kDeWarps * 32), args, smem, st));
   return SEMB_OK;
 }

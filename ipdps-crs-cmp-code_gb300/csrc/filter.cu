@@ -79,10 +79,10 @@ bool filter_exists(int form, int w, int brun, int pipe, int lay) {
 }
 
 // Once per plan configuration, before its launches (which may be captured).
-int filter_prepare(int form, int w, int storage, int shape, size_t smem) {
+int filter_prepare(int form, int w, int storage, int shape) {
   const void* fn = filter_fn(form, w, storage, shape);
   if (!fn) return fail(SEMB_E_WINDOW, "no filter kernel for w = %d", w);
-  SEMB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SEMB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem));
   return SEMB_OK;
 }
 

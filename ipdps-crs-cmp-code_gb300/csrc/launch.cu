@@ -146,7 +146,9 @@ int fallback_variant(int method, int form, int w, int nb) {
 int search_occupancy(int method, int form, int w, int v, int nwarps, size_t smem, int* ctas_per_sm) {
   SearchEntry e = lookup(method, form, w, v);
   if (!e.fn) return fail(SEMB_E_WINDOW, "no search kernel for w = %d", w);
-  SEMB_CUDA(cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the most any plan takes: the limit belongs to the kernel, and live plans of other sizes
+  // (a ring kernel's depends on the candidate count) launch it too
+  SEMB_CUDA(cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem));
   SEMB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, e.fn, nwarps * 32, smem));
   return SEMB_OK;
 }

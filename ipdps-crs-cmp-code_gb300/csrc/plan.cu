@@ -56,7 +56,7 @@ int launch_crs_de(int w, const DeParams& R, KParams P, cudaStream_t st);
 bool filter_exists(int form, int w, int brun, int pipe, int lay);
 int filter_shape(int w, int nb, int* rc, int* nt);
 size_t filter_smem(int form, int storage, int nt, int cap);
-int filter_prepare(int form, int w, int storage, int shape, size_t smem);
+int filter_prepare(int form, int w, int storage, int shape);
 int launch_filter(int form, int w, int storage, int shape, const FilterParams& F, int nwarps, int grid, size_t smem,
                   cudaStream_t st);
 int launch_refine(int form, int w, int lay, const RefineParams& R, cudaStream_t st);
@@ -561,7 +561,7 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(f.d_pass_bounds, bounds.data(), bounds.size() * 4, cudaMemcpyHostToDevice, pl->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(pl->stream);
-  int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, shape, f.smem) : SEMB_OK;
+  int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, shape) : SEMB_OK;
   if (e != cudaSuccess || rc_prep != SEMB_OK) {
     dev_free(f.d_cand);
     dev_free(f.d_pass_bounds);
@@ -665,8 +665,8 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   };
   // the ring kernels' CTAs share the SM only where each still holds a whole trace's window
   // in every plane
-  while (pipe >= 3 && minb > 1 && smem_of((int)pl->pitch + 16) > (227 * 1024) / (size_t)minb - 1024) --minb;
-  const size_t budget = (227 * 1024) / minb - 1024;
+  while (pipe >= 3 && minb > 1 && smem_of((int)pl->pitch + 16) > kMaxDynamicSmem / (size_t)minb - 1024) --minb;
+  const size_t budget = kMaxDynamicSmem / minb - 1024;
   int cap = form == FORM_PLAIN || pipe == 4 ? 32768 : 8192;
   if (form == FORM_FAST && pl->stage_cap > 0) cap = std::min(cap, pl->stage_cap);
   if (lay == LAY_X3) cap = std::min(cap, kXPlane - kZeroSlots);
@@ -675,7 +675,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   if (small_stages) min_cap = std::min(min_cap, pl->stage_cap > 0 ? pl->stage_cap : kMinStage);
   if (cap < min_cap) cap = (min_cap + 63) & ~63;
   const size_t smem = smem_of(cap);
-  if (smem > 227 * 1024) return fail(SEMB_E_ARG, "ns %d too large for the staging buffer", pl->ns);
+  if (smem > kMaxDynamicSmem) return fail(SEMB_E_ARG, "ns %d too large for the staging buffer", pl->ns);
   int occ = 0;
   SEMB_TRY(search_occupancy(p.method, form, pl->w, v, best_nw, smem, &occ));
   if (occ <= 0) return fail(SEMB_E_CUDA, "search kernel cannot be resident with %zu bytes", smem);
