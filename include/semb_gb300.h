@@ -328,6 +328,21 @@ int semb_plan_set_variant(semb_plan* plan, int32_t variant);
  * counterpart in the reference. */
 int semb_plan_set_staging(semb_plan* plan, int32_t max_samples);
 
+/* The CRS grid search's filter, which bounds every candidate and evaluates only the few
+ * that can win (both forms): SEMB_FILTER_AUTO, the default, uses it where it pays,
+ * SEMB_FILTER_OFF evaluates every candidate, SEMB_FILTER_ON uses it wherever the plan's
+ * window, grid, record and kernel variant have one, whatever it costs.  The filter's
+ * bounds allow for FP32 rounding as a multiple of its rms: the results are those of the
+ * search without it unless a candidate's rounding exceeds that.  Takes effect at once on
+ * an uploaded plan and stays for later uploads.  No counterpart in the reference. */
+enum { SEMB_FILTER_OFF = 0, SEMB_FILTER_AUTO = 1, SEMB_FILTER_ON = 2 };
+int semb_plan_set_filter(semb_plan* plan, int32_t mode);
+
+/* The filter's use (either pointer may be NULL): *filtered gets the tasks (CDP x 32-sample
+ * t0 blocks) that a run searches through it (0: no filter), *direct the tasks of the last
+ * run that it handed to the direct kernel because too many candidates were close. */
+int semb_plan_filter_tasks(semb_plan* plan, int64_t* filtered, int64_t* direct);
+
 /* Batched grid search in chunks of cdps_per_chunk contiguous CDPs (0, the default:
  * the whole survey at once).  semb_plan_run then searches the chunks one after the
  * other; each chunk's work (the CRS t0 = 0 stacks, one search launch per run of

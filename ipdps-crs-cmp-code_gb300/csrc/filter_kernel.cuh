@@ -97,6 +97,7 @@ struct FilterParams {
   unsigned long long* pool_count;
   int2* fb_tasks;          // tasks whose lists overflowed
   int* fb_count;
+  unsigned long long* fb_total;   // counts them over all launches of a run
   float kappa;             // multiple of the rms rounding effect (see above)
 };
 
@@ -858,7 +859,10 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
           const bool fb = __any_sync(0xffffffffu, over);
           if (in) FP.head[(int64_t)tg.cdp * P.ns + tt] = make_int2(base + incl - cnt, fb ? -1 : cnt);
           if (fb) {
-            if (lane == 0) FP.fb_tasks[atomicAdd(FP.fb_count, 1)] = make_int2(tg.cdp, tg.t0s);
+            if (lane == 0) {
+              FP.fb_tasks[atomicAdd(FP.fb_count, 1)] = make_int2(tg.cdp, tg.t0s);
+              atomicAdd(FP.fb_total, 1ull);
+            }
           } else if (cnt > 0) {
             int2* out = FP.pool + base + incl - cnt;
             for (int w2 = 0; w2 < nwarps; ++w2)

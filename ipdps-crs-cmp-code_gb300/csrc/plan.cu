@@ -152,12 +152,14 @@ struct semb_plan {
   float* d_top_stk = nullptr;
   // CRS filter: the kept runs (per (CDP, t0) their place in a pool); overflowed tasks;
   // {their count, their queue head, the filter's queue head, -, the pool's entries (64
-  // bits)}, zeroed before every filter launch
+  // bits)}, zeroed before every filter launch, and the run's overflowed tasks (64 bits),
+  // zeroed before every run
   int2* d_head = nullptr;
   int2* d_pool = nullptr;
   int pool_cap = 0;
   int2* d_fb_tasks = nullptr;
   int* d_fb_count = nullptr;
+  int filter_mode = SEMB_FILTER_AUTO;
   int* d_status = nullptr;
   unsigned long long* d_repicked = nullptr;
   // extra attributes (batched form with attrs = 1)
@@ -466,7 +468,9 @@ float4 sample_candidate(const semb_plan* pl, int gi, bool pad) {
 int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_direct, KernelCfg& c) {
   const semb_params& p = pl->p;
   const int form = p.mode == SEMB_PLAIN_F32 ? FORM_PLAIN : FORM_FAST;
-  if (p.method != SEMB_CRS || p.ngen > 0 || p.nb < 2 || !filter_exists(form, pl->w, brun, pipe, lay)) return SEMB_OK;
+  if (pl->filter_mode == SEMB_FILTER_OFF || p.method != SEMB_CRS || p.ngen > 0 || p.nb < 2 ||
+      !filter_exists(form, pl->w, brun, pipe, lay))
+    return SEMB_OK;
   int rc = 0, nt = 0;
   const int shape = filter_shape(pl->w, p.nb, &rc, &nt), cs = (rc - 1) / 2;
   const int nruns = (p.nb + rc - 1) / rc;
@@ -478,7 +482,7 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   // 7 x 21 x 7 grid with little more than one task per SM 1.5 and 1.3.
   const double direct = (form == FORM_PLAIN ? 73.0 : 25.0 + (pl->w == 5 ? 8.0 : 0.0)) * (double)pl->ncand;
   const double filtered = (100.0 + 3.5 * rc) * (double)total + (form == FORM_PLAIN ? 3500.0 : 8600.0);
-  if (filtered > 0.9 * direct) return SEMB_OK;
+  if (filtered > 0.9 * direct && pl->filter_mode != SEMB_FILTER_ON) return SEMB_OK;
   // each (A, C) group's B values cut into the fewest runs of at most rc, of equal length
   // give or take one, each run's middle value in slot cs, B ascending with the slot; padding
   // repeats the run's ends
@@ -550,7 +554,7 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
     dev_release(pl, pl->d_fb_tasks);
     return SEMB_OK;
   }
-  if (dev_reuse(pl, &pl->d_fb_count, 6, true) != SEMB_OK || dev_alloc(&f.d_cand, npad) != SEMB_OK ||
+  if (dev_reuse(pl, &pl->d_fb_count, 8, true) != SEMB_OK || dev_alloc(&f.d_cand, npad) != SEMB_OK ||
       dev_alloc(&f.d_pass_bounds, bounds.size()) != SEMB_OK) {
     cudaGetLastError();
     dev_free(f.d_cand);
@@ -560,6 +564,7 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_dir
   cudaError_t e = cudaMemcpyAsync(f.d_cand, cand.data(), npad * sizeof(float4), cudaMemcpyHostToDevice, pl->stream);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(f.d_pass_bounds, bounds.data(), bounds.size() * 4, cudaMemcpyHostToDevice, pl->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(pl->d_fb_count, 0, 8 * sizeof(int), pl->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(pl->stream);
   int rc_prep = e == cudaSuccess ? filter_prepare(form, pl->w, store, shape) : SEMB_OK;
   if (e != cudaSuccess || rc_prep != SEMB_OK) {
@@ -1363,6 +1368,7 @@ int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int n
     F.pool_count = reinterpret_cast<unsigned long long*>(pl->d_fb_count + 4);
     F.fb_tasks = pl->d_fb_tasks;
     F.fb_count = pl->d_fb_count;
+    F.fb_total = reinterpret_cast<unsigned long long*>(pl->d_fb_count + 6);
     F.kappa = form == FORM_PLAIN ? 16.f : 8.f;
     SEMB_TRY(launch_filter(form, pl->w, P.storage, f->shape, F, f->nwarps, std::min(ntasks, pl->sms), f->smem, st));
     RefineParams R{};
@@ -1386,6 +1392,16 @@ int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int n
   }
   SEMB_TRY(launch_search(p.method, form, pl->w, cfg.variant, P, cfg.nwarps, grid, cfg.smem, st));
   if (launches) ++*launches;
+  return SEMB_OK;
+}
+
+// Before a run: no task handed over by the filter yet.
+int reset_filter_total(semb_plan* pl) {
+  for (const Bucket& b : pl->buckets)
+    if (b.cfg.filter) {
+      SEMB_CUDA(cudaMemsetAsync(pl->d_fb_count + 6, 0, 2 * sizeof(int), pl->stream));
+      break;
+    }
   return SEMB_OK;
 }
 
@@ -1540,6 +1556,7 @@ int enqueue_streamed(semb_plan* pl, const semb_gather_view* g) {
   SEMB_TRY(dev_reuse(pl, &pl->d_chunk_counter, nk));
   SEMB_CUDA(cudaMemsetAsync(pl->d_status, 0, kStatusWords * sizeof(int), st));
   SEMB_CUDA(cudaMemsetAsync(pl->d_chunk_counter, 0, nk * sizeof(int), st));
+  SEMB_TRY(reset_filter_total(pl));
   SEMB_CUDA(cudaEventRecord(pl->ev[0], st));
   const Bucket& b = pl->buckets[0];
   int launches = 0;
@@ -1741,6 +1758,32 @@ int semb_plan_set_staging(semb_plan* pl, int32_t max_samples) {
   return SEMB_OK;
 }
 
+int semb_plan_set_filter(semb_plan* pl, int32_t mode) {
+  if (!pl) return fail(SEMB_E_ARG, "null argument");
+  if (mode < SEMB_FILTER_OFF || mode > SEMB_FILTER_ON) return fail(SEMB_E_ARG, "unknown filter mode %d", mode);
+  pl->filter_mode = mode;
+  if (!pl->uploaded) return SEMB_OK;
+  SEMB_CUDA(cudaSetDevice(pl->device));
+  for (Bucket& b : pl->buckets) SEMB_TRY(build_cfg(pl, b.cfg.variant, b.cfg));
+  refresh_stats(pl);
+  return SEMB_OK;
+}
+
+int semb_plan_filter_tasks(semb_plan* pl, int64_t* filtered, int64_t* direct) {
+  if (!pl) return fail(SEMB_E_ARG, "null argument");
+  if (!pl->uploaded) return fail(SEMB_E_STATE, "semb_plan_filter_tasks before semb_plan_upload");
+  int64_t n = 0;
+  for (const Bucket& b : pl->buckets)
+    if (b.cfg.filter) n += b.end - b.begin;
+  if (filtered) *filtered = n;
+  if (direct) {
+    *direct = 0;
+    SEMB_CUDA(cudaSetDevice(pl->device));
+    if (n > 0) SEMB_CUDA(cudaMemcpy(direct, pl->d_fb_count + 6, sizeof(*direct), cudaMemcpyDeviceToHost));
+  }
+  return SEMB_OK;
+}
+
 int semb_plan_use_graph(semb_plan* pl, int32_t on) {
   if (!pl) return fail(SEMB_E_ARG, "null argument");
   pl->use_graph = on != 0;
@@ -1757,6 +1800,7 @@ int semb_plan_run(semb_plan* pl) {
   SEMB_CUDA(cudaSetDevice(pl->device));
   cudaStream_t st = pl->stream;
   SEMB_CUDA(cudaMemsetAsync(pl->d_status, 0, kStatusWords * sizeof(int), st));
+  SEMB_TRY(reset_filter_total(pl));
   const bool chunked = pl->chunk_cdps > 0 && pl->p.mode == SEMB_BATCHED && pl->p.ngen == 0 &&
                        pl->ns >= 2 * pl->tau + 2;
   pl->chunk_ms.clear();

@@ -31,6 +31,7 @@ PLAIN_F32, BATCHED = 0, 1
 STORE_F32, STORE_F16, STORE_BF16 = 0, 1, 2
 REPICK_OFF, REPICK_NEAR_TIES, REPICK_ALWAYS = 0, 1, 2
 DM_ABS, DM_SIGNED = 0, 1
+FILTER_OFF, FILTER_AUTO, FILTER_ON = 0, 1, 2
 ABI_VERSION = 9
 MAX_VARIANTS = 34   # SEMB_MAX_VARIANTS
 MAX_BUCKETS = 4     # SEMB_MAX_BUCKETS
@@ -43,7 +44,7 @@ EXPORTS = [
     "semb_plan_download", "semb_plan_download_attrs", "semb_survey_write_attr", "semb_plan_download_abc",
     "semb_survey_write_abc", "semb_plan_neighbours", "semb_neighbours_noalloc", "semb_plan_stats",
     "semb_plan_autotune", "semb_plan_buckets", "semb_plan_set_variant", "semb_plan_set_staging",
-    "semb_plan_set_chunks", "semb_plan_chunk_times",
+    "semb_plan_set_filter", "semb_plan_filter_tasks", "semb_plan_set_chunks", "semb_plan_chunk_times",
     "semb_plan_use_graph", "semb_plan_destroy",
     "semb_host_alloc", "semb_host_free", "semb_probe_fp32", "semb_selftest_wait", "semb_device_count",
     "semb_strerror", "semb_last_error", "semb_abi_version",
@@ -127,6 +128,8 @@ def lib():
         "semb_plan_buckets": (C.c_int, [P, P, P, P, P, P]),
         "semb_plan_set_variant": (C.c_int, [P, i32]),
         "semb_plan_set_staging": (C.c_int, [P, i32]),
+        "semb_plan_set_filter": (C.c_int, [P, i32]),
+        "semb_plan_filter_tasks": (C.c_int, [P, P, P]),
         "semb_plan_set_chunks": (C.c_int, [P, i32]),
         "semb_plan_chunk_times": (C.c_int, [P, i32, P, P]),
         "semb_plan_use_graph": (C.c_int, [P, i32]),
@@ -365,6 +368,18 @@ class Plan:
 
     def set_variant(self, v: int) -> None:
         _check(lib().semb_plan_set_variant(self._h, int(v)), "semb_plan_set_variant")
+
+    def set_filter(self, mode: int) -> None:
+        """CRS grid search: FILTER_OFF evaluates every candidate, FILTER_AUTO (the default)
+        filters them where that pays, FILTER_ON wherever a filter applies."""
+        _check(lib().semb_plan_set_filter(self._h, int(mode)), "semb_plan_set_filter")
+
+    def filter_tasks(self):
+        """(tasks searched through the filter, those of the last run that it handed to the
+        direct kernel)."""
+        n, d = C.c_int64(), C.c_int64()
+        _check(lib().semb_plan_filter_tasks(self._h, C.byref(n), C.byref(d)), "semb_plan_filter_tasks")
+        return int(n.value), int(d.value)
 
     def set_chunks(self, cdps_per_chunk: int) -> None:
         """Run the batched grid search in chunks of contiguous CDPs, each chunk's

@@ -1,0 +1,191 @@
+"""The CRS filter against the search without it (GPU).  Every test asserts that the filter is
+attached, turns it off on the same plan and compares the results bit for bit: the refine's
+arithmetic is the direct kernel's, and what the filter leaves out must not have won.
+Windows, stores, runs of every slot count, several runs per (A, C), padding, descending B,
+early samples (whose runs do not expand), records that the traces leave, apertures where
+everything ties, streamed, chunked and graph runs."""
+import numpy as np
+import pytest
+
+import oracle
+import semb
+import synth
+
+pytestmark = pytest.mark.gpu
+
+STORES = {"f32": semb.STORE_F32, "f16": semb.STORE_F16, "bf16": semb.STORE_BF16}
+
+
+def _survey(nb, tau, ns=600, apm=50, b1=1e-7, ncdp=9, fold=9, na=5, nc=5, az=0.0, seed=0):
+    s = synth.crs_survey(seed=800 + nb + seed, ncdp=ncdp, noffsets=fold, ns=ns, na=na, nb=nb, nc=nc,
+                         tau=tau * 0.002 * 1.0001, apm=apm, azimuth=az)
+    s.params["b0"], s.params["b1"] = -b1, b1
+    return s
+
+
+def _arrays(s):
+    g = oracle.gather(s.headers, s.samples, "crs", s.params["aph"], s.params["apm"], real=np.float32)
+    return semb.GatherArrays(g["ntraces_by_cdp_id"], g["ns"], g["dt_us"], g["gx"], g["gy"], g["sx"], g["sy"],
+                             g["scalco"], g["samples"])
+
+
+def _kw(form, signed=False, **kw):
+    kw["dm_mode"] = semb.DM_SIGNED if signed else semb.DM_ABS
+    if form == "plain":
+        return dict(mode=semb.PLAIN_F32, **kw)
+    return dict(mode=semb.BATCHED, storage=STORES[form], repick=semb.REPICK_OFF, attrs=1, **kw)
+
+
+def _results(p, form):
+    p.run()
+    out = list(p.download())
+    if form != "plain":
+        a = p.download_attrs()
+        out += [a["sem2"], a["idx2"]]
+    return out
+
+
+def _compare(s, form, overflow=None, variant=None, **kw):
+    """Filtered and unfiltered results of one plan; returns the unfiltered ones."""
+    arr = _arrays(s)
+    with semb.Plan(semb.params(semb.CRS, **_kw(form, **kw), **s.params)) as p:
+        p.set_filter(semb.FILTER_ON)
+        p.upload(arr.view())
+        if variant is not None:
+            p.set_variant(variant)
+        tasks = p.filter_tasks()[0]
+        assert tasks == p.ncdps * ((p.ns + 31) // 32)
+        got = _results(p, form)
+        direct = p.filter_tasks()[1]
+        assert 0 <= direct <= tasks
+        if overflow is not None:
+            assert (direct > 0) == overflow, (direct, tasks)
+        p.set_filter(semb.FILTER_OFF)
+        assert p.filter_tasks() == (0, 0)
+        ref = _results(p, form)
+    for x, y in zip(got, ref):
+        assert np.array_equal(x, y, equal_nan=x.dtype.kind == "f"), np.mean(x != y)
+    return ref
+
+
+# slots of 8 to 32 and their neighbours, two and three runs per (A, C)
+RUNS = [(2, 1), (12, 1), (13, 1), (16, 1), (17, 1), (21, 1), (22, 1), (23, 1), (31, 1), (32, 1), (33, 1), (45, 1),
+        (70, 1), (8, 2), (9, 2), (13, 2), (14, 2), (15, 2), (22, 2), (25, 2), (47, 2)]
+
+
+@pytest.mark.parametrize("form", ["plain", "f16", "bf16", "f32"])
+@pytest.mark.parametrize("nb,tau", RUNS)
+def test_runs_of_every_length(nb, tau, form):
+    ref = _compare(_survey(nb, tau, ns=601 if nb % 2 else 608, na=3), form)
+    assert np.mean(ref[1] > 0) > 0.5
+
+
+@pytest.mark.parametrize("nb", [3, 12, 31, 40])
+def test_one_sample_windows(nb):
+    _compare(_survey(nb, 0, ns=610), "plain")
+
+
+@pytest.mark.parametrize("form", ["plain", "f16", "f32"])
+@pytest.mark.parametrize("case", [dict(b1=-1e-7), dict(b1=2e-7), dict(b1=4e-8, ns=300), dict(apm=100, b1=4e-8),
+                                  dict(fold=40, ncdp=5, ns=650), dict(ncdp=1, fold=3)],
+                         ids=str)
+@pytest.mark.parametrize("signed", [False, True])
+@pytest.mark.parametrize("tau", [1, 2])
+def test_geometries(case, form, signed, tau):
+    _compare(_survey(21, tau, az=30.0 if signed else 0.0, **case), form, signed=signed)
+
+
+@pytest.mark.parametrize("variant", [10, 13, 14, 28, 30, 31, 32, 33])
+def test_every_filtered_variant(variant):
+    s = _survey(21, 1)
+    arr = _arrays(s)
+    with semb.Plan(semb.params(semb.CRS, **_kw("f16"), **s.params)) as p:
+        p.set_filter(semb.FILTER_ON)
+        p.upload(arr.view())
+        p.set_variant(variant)
+        if p.filter_tasks()[0] == 0:
+            assert variant == 10   # a kernel without the pipelined staging
+            return
+    _compare(s, "f16", variant=variant)
+
+
+@pytest.mark.parametrize("form", ["plain", "f16", "bf16", "f32"])
+def test_apertures_of_one_cdp_overflow_into_the_direct_kernel(form):
+    """Every A and B ties: no list holds them all."""
+    _compare(_survey(21, 1, apm=5, ncdp=3, na=9), form, overflow=True)
+
+
+@pytest.mark.parametrize("form", ["plain", "f16", "f32"])
+def test_no_valid_candidate(form):
+    s = _survey(21, 1)
+    s.params["c0"] *= 400.0
+    s.params["c1"] *= 400.0
+    ref = _compare(s, form, overflow=False)
+    assert np.any(ref[1] == 0)
+
+
+@pytest.mark.parametrize("form", ["plain", "f32"])
+def test_zero_and_non_finite_traces(form):
+    s = _survey(21, 1)
+    s.samples[3] = 0.0
+    s.samples[20, 100] = np.inf
+    s.samples[41, 150] = np.nan
+    s.samples[60] *= 1e-12
+    s.samples[:, 400:430] = 0.0
+    _compare(s, form)
+
+
+@pytest.mark.parametrize("form", ["f16", "f32"])
+@pytest.mark.parametrize("tau", [1, 2])
+def test_streamed_chunked_and_graph_runs(form, tau):
+    s = _survey(21, tau, ncdp=14)
+    arr = _arrays(s)
+    with semb.Plan(semb.params(semb.CRS, **_kw(form), **s.params)) as p:
+        p.set_filter(semb.FILTER_OFF)
+        p.upload(arr.view())
+        ref = _results(p, form)[:3]
+
+        def same():
+            assert p.filter_tasks()[0] > 0
+            for x, y in zip(p.download(), ref):
+                assert np.array_equal(x, y)
+
+        p.set_filter(semb.FILTER_ON)
+        for _ in range(2):   # captured, replayed
+            p.use_graph(True)
+            p.run()
+            same()
+        p.use_graph(False)
+        for _ in range(2):
+            p.set_chunks(4)
+            p.run()
+            same()
+        p.set_chunks(0)
+        p.stream(arr.view(), 3)
+        same()
+
+
+@pytest.mark.parametrize("form", ["plain", "f16"])
+def test_default_use(form):
+    """Where it pays: the 21 x 21 x 21 grid, not a 3 x 3 x 3 one or one B value, never CMP."""
+    def tasks(**kw):
+        s = _survey(ns=600, tau=1, ncdp=3, **kw)
+        with semb.Plan(semb.params(semb.CRS, **_kw(form), **s.params)) as p:
+            p.upload(_arrays(s).view())
+            return p.filter_tasks()[0]
+
+    assert tasks(na=21, nb=21, nc=21) > 0
+    assert tasks(na=3, nb=3, nc=3) == 0
+    assert tasks(na=21, nb=1, nc=21) == 0
+    s = synth.cmp_survey(seed=1, ncmp=2, half_offsets=np.linspace(10.0, 300.0, 20), ns=320, nc=64, tau=0.0021)
+    g = oracle.gather(s.headers, s.samples, "cmp", s.params["aph"])
+    arr = semb.GatherArrays(g["ntraces_by_cdp_id"], g["ns"], g["dt_us"], g["gx"], g["gy"], g["sx"], g["sy"],
+                            g["scalco"], g["samples"])
+    with semb.Plan(semb.params(semb.CMP, mode=semb.PLAIN_F32, **s.params)) as p:
+        with pytest.raises(semb.SembError):
+            p.filter_tasks()   # before the upload
+        with pytest.raises(semb.SembError):
+            p.set_filter(3)
+        p.set_filter(semb.FILTER_ON)
+        p.upload(arr.view())
+        assert p.filter_tasks() == (0, 0)
