@@ -147,11 +147,12 @@ static __device__ __noinline__ void central_add(const KParams& P, int t0s, int64
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const uint32_t b = __ldg(P.samples16 + at + u);
-          v[u] = (P.storage == STORE_F16 ? half_bits_to_float(b) : __uint_as_float(b << 16)) * sc;
+          v[u] = __fmul_rn(P.storage == STORE_F16 ? half_bits_to_float(b) : __uint_as_float(b << 16), sc);
         }
       }
-      // the packed value/difference entry (s_0, s_2, d_0, d_2) and its window
-      const float d0 = v[1] - v[0], d2 = v[3] - v[2];
+      // the packed value/difference entry (s_0, s_2, d_0, d_2) and its window; the
+      // differences are of the rounded values (the refine kernel repeats them)
+      const float d0 = __fsub_rn(v[1], v[0]), d2 = __fsub_rn(v[3], v[2]);
       const float w0 = fmaf(d0, x, v[0]), w2 = fmaf(d2, x, v[2]);
       const float s1 = v[0] + d0;
       const float w1 = fmaf(v[2] - s1, x, s1);

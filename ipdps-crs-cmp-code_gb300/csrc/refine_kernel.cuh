@@ -181,9 +181,9 @@ __global__ void __launch_bounds__(256) k_refine_plain(RefineParams R) {
 // ---- batched form -----------------------------------------------------------------
 
 // Window samples s_0 .. s_W at sample rel of trace tr as the staging converts them, and the
-// differences of the LAY_PD entry.  CT: the differences take the scale in one rounding
-// (the compiler contracts convert_chunk's v[1] - v[0] into h[1] * scale - v[0]); the
-// central traces' sums (central_add) form them from two rounded samples.
+// differences of the LAY_PD entry.  CT: the differences take the scale in one rounding, as
+// convert_chunk forms them; the central traces' sums (central_add) take them of two rounded
+// samples.
 template <int W, bool CT>
 __device__ __forceinline__ void store_samples(const KParams& P, int tr, int rel, float (&s)[W + 8], float& d0,
                                               float& d2) {
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) k_refine_fast(RefineParams R) {
     ze = zb + zr.y;
   }
   const float T = (float)t0;
-  const float T_lo = P.dt * (float)td.y, T_hi = P.dt * (float)min(td.y + kTB - 1, P.ns - 1);
+  const float T_lo = __fmul_rn(P.dt, (float)td.y), T_hi = __fmul_rn(P.dt, (float)min(td.y + kTB - 1, P.ns - 1));
   const unsigned span = (unsigned)(P.ns - 2 * P.tau - 2);
   float fs[kTopK] = {}, fk[kTopK] = {};
   int fi[kTopK];

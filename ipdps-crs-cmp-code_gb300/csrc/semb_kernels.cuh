@@ -340,7 +340,9 @@ __host__ __device__ inline SmemLayout smem_layout(int form, int rc, int cap, int
 // Sample window [lo, hi] of one trace that items of a pass can read, for t0 in
 // [T_lo, T_hi] (seconds) and parameters within the pass bounds.  Returns false
 // when no item can be in range: then the trace is left out of the chunk, which is
-// exact, because an out-of-range trace only counts in err = N_ap - M.
+// exact, because an out-of-range trace only counts in err = N_ap - M.  Every operation is
+// written out: the refine kernels repeat a planner's chunks from it, and a sum that one
+// caller's compilation contracts with what surrounds it would move a window's end there.
 template <int METHOD>
 __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_lo, float T_hi, float idt,
                                              int tau, int ns, int& lo, int& hi, bool& inrange, float& smin) {
@@ -348,21 +350,22 @@ __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_
   float t2min, t2max;
   if (METHOD == METHOD_CMP) {
     // t^2 = t0^2 + c*h, h >= 0
-    t2min = T_lo * T_lo + fminf(pb[4] * g.z, pb[5] * g.z);
-    t2max = T_hi * T_hi + fmaxf(pb[4] * g.z, pb[5] * g.z);
+    const float c0 = __fmul_rn(pb[4], g.z), c1 = __fmul_rn(pb[5], g.z);
+    t2min = __fmaf_rn(T_lo, T_lo, fminf(c0, c1));
+    t2max = __fmaf_rn(T_hi, T_hi, fmaxf(c0, c1));
   } else {
     // t^2 = (t0 + a*m)^2 + b*m2 + c*h with m2, h >= 0; m >= 0, or signed along the
     // azimuth
-    const float am0 = pb[0] * g.x, am1 = pb[1] * g.x;
-    float ulo = T_lo + fminf(am0, am1), uhi = T_hi + fmaxf(am0, am1);
-    float u2lo = (ulo <= 0.f && uhi >= 0.f) ? 0.f : fminf(ulo * ulo, uhi * uhi);
-    float u2hi = fmaxf(ulo * ulo, uhi * uhi);
-    t2min = u2lo + pb[2] * g.y + pb[4] * g.z;
-    t2max = u2hi + pb[3] * g.y + pb[5] * g.z;
+    const float am0 = __fmul_rn(pb[0], g.x), am1 = __fmul_rn(pb[1], g.x);
+    const float ulo = __fadd_rn(T_lo, fminf(am0, am1)), uhi = __fadd_rn(T_hi, fmaxf(am0, am1));
+    const float l2 = __fmul_rn(ulo, ulo), h2 = __fmul_rn(uhi, uhi);
+    const float u2lo = (ulo <= 0.f && uhi >= 0.f) ? 0.f : fminf(l2, h2);
+    t2min = __fmaf_rn(pb[4], g.z, __fmaf_rn(pb[2], g.y, u2lo));
+    t2max = __fmaf_rn(pb[5], g.z, __fmaf_rn(pb[3], g.y, fmaxf(l2, h2)));
   }
   // relative slack for rounding differences between this bound and the items
-  t2min -= fabsf(t2min) * 1e-5f;
-  t2max += fabsf(t2max) * 1e-5f;
+  t2min = __fmaf_rn(fabsf(t2min), -1e-5f, t2min);
+  t2max = __fmaf_rn(fabsf(t2max), 1e-5f, t2max);
   if (!(t2max >= 0.f)) {
     // every item has a negative t^2 (or the bound is not finite): nothing in range
     if (t2max < 0.f) return false;
@@ -370,8 +373,8 @@ __device__ __forceinline__ bool trace_window(const float* pb, float4 g, float T_
     hi = ns - 1;
     return true;
   }
-  smin = t2min > 0.f ? sqrtf(t2min) * idt : 0.f;
-  float smax = sqrtf(t2max) * idt;
+  smin = t2min > 0.f ? __fmul_rn(__fsqrt_rn(t2min), idt) : 0.f;
+  float smax = __fmul_rn(__fsqrt_rn(t2max), idt);
   smin = fminf(smin, (float)ns + 8.f);
   smax = fminf(smax, (float)ns + 8.f);
   // in range for sure: tau <= it <= ns - tau - 2 for every item, with one sample of slack
@@ -614,24 +617,28 @@ __device__ __forceinline__ void convert_chunk(const KParams& P, const ChunkMeta*
       continue;
     }
     for (int k = lane; k < si.z; k += 32) {
-      float v[4];
+      // stored samples h, values v = h * sc; a difference d_j takes the scale in one rounding
+      // (fma(h_j+1, sc, -v_j)), which the refine kernels repeat (store_samples)
+      float h[4], v[4];
 #pragma unroll
       for (int u = 0; u < (LAY == LAY_SD ? 3 : 4); ++u) {
         if (P.storage == STORE_F32) {
-          v[u] = r32[k + u];
+          h[u] = r32[k + u];
         } else {
           const uint32_t b = r16[k + u];
-          v[u] = (f16 ? half_bits_to_float(b) : __uint_as_float(b << 16)) * sc;
+          h[u] = f16 ? half_bits_to_float(b) : __uint_as_float(b << 16);
         }
+        v[u] = __fmul_rn(h[u], sc);
       }
+      auto diff = [&](int j) { return __fmaf_rn(h[j + 1], sc, -v[j]); };
       constexpr int SL = stage_lay(LAY);
-      dst[k] = SL == LAY_SD   ? make_float4(v[0], v[1] - v[0], v[1], v[2] - v[1])
+      dst[k] = SL == LAY_SD   ? make_float4(v[0], diff(0), v[1], diff(1))
                : SL == LAY_P2 ? make_float4(v[0], v[2], v[1], v[3])
-               : (SL == LAY_PD || SL == LAY_PD5) ? make_float4(v[0], v[2], v[1] - v[0], v[3] - v[2])
+               : (SL == LAY_PD || SL == LAY_PD5) ? make_float4(v[0], v[2], diff(0), diff(2))
                                                  : make_float4(v[0], v[1], v[2], v[3]);
       if constexpr (SL == LAY_PD5) {
         // side entry (s_k, d_k), after the main entries and their zero block
-        reinterpret_cast<float2*>(bufq + P.cap + kZeroSlots)[si.w + k] = make_float2(v[0], v[1] - v[0]);
+        reinterpret_cast<float2*>(bufq + P.cap + kZeroSlots)[si.w + k] = make_float2(v[0], diff(0));
       }
     }
   }

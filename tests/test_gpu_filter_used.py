@@ -95,6 +95,14 @@ def test_geometries(case, form, signed, tau):
     _compare(_survey(21, tau, az=30.0 if signed else 0.0, **case), form, signed=signed)
 
 
+@pytest.mark.parametrize("form", ["f16", "bf16", "f32"])
+@pytest.mark.parametrize("seed", range(4))
+@pytest.mark.parametrize("tau", [1, 2])
+def test_chunks_end_where_the_direct_kernel_s_do(tau, seed, form):
+    """Folds of several staged chunks: the refine folds its energies at the same traces."""
+    _compare(_survey(21, tau, az=30.0, ncdp=25, fold=17, ns=777, seed=seed), form, signed=True)
+
+
 @pytest.mark.parametrize("variant", [10, 13, 14, 28, 30, 31, 32, 33])
 def test_every_filtered_variant(variant):
     s = _survey(21, 1)
