@@ -285,8 +285,8 @@ struct ChunkMeta {
                            // [kMaxChunk - (n - n_in), kMaxChunk).  Plain form: n_in = n
   int consumed;            // aperture traces the chunk covers (entries + skipped)
   int bytes;               // bytes staged (TMA form)
-  int quad;                // semb_filter_kernel: some in-range entry needs the expansion's
-                           // second-order terms
+  int quad;                // semb_filter_kernel: some entry whose run expands needs the
+                           // expansion's second-order terms
 };
 
 constexpr size_t kMetaBytes = ((sizeof(ChunkMeta) + 127) / 128) * 128;
@@ -494,7 +494,8 @@ __device__ void plan_chunk(const KParams& P, const float* pb, int64_t ap_pos, in
       else meta->raw[e] = glob ? tr : off + 8 * rank;
       src[e] = make_int4(tr, lo, len, off);   // len 0: nothing to copy or convert
     }
-    if constexpr (MOM) quad = quad || __any_sync(0xffffffffu, take && front && !linear);
+    // (a narrow trace in the back part joins the moments and the crossings too)
+    if constexpr (MOM) quad = quad || __any_sync(0xffffffffu, take && kind == 1 && !linear);
     const int nhave = __popc(__ballot_sync(0xffffffffu, have));
     base += stop > 0 ? __shfl_sync(0xffffffffu, incl, stop - 1) : 0;
     n_in += __popc(fr);

@@ -103,6 +103,57 @@ def test_chunks_end_where_the_direct_kernel_s_do(tau, seed, form):
     _compare(_survey(21, tau, az=30.0, ncdp=25, fold=17, ns=777, seed=seed), form, signed=True)
 
 
+class _Scattered:
+    """Pairs of CDPs 1 km apart.  The second CDP's traces, `nfar` of them, lie far from its
+    first trace's midpoint, with offsets that take them to the record's end: their runs are
+    wide, their expansion needs its second order, and no other trace of a chunk does."""
+
+    def __init__(self, seed, npairs=48, nnear=2, nfar=400, ns=300, far=105, spread=0):
+        r = np.random.default_rng(seed)
+        n = npairs * (nnear + 1 + nfar)
+        self.ns, self.ncdp = ns, 2 * npairs
+        mx, half = np.empty(n), np.empty(n)
+        end, q = [], 0
+        for k in range(npairs):
+            mx[q:q + nnear] = 1000 * k
+            half[q:q + nnear] = 20
+            q += nnear
+            end.append(q)
+            mx[q] = 1000 * k + 49
+            half[q] = 20
+            mx[q + 1:q + 1 + nfar] = 1000 * k + far + r.integers(-spread, spread + 1, nfar)
+            half[q + 1:q + 1 + nfar] = 320 + r.integers(-spread, spread + 1, nfar)
+            q += 1 + nfar
+            end.append(q)
+        self.sx, self.gx = (mx - half).astype(np.int32), (mx + half).astype(np.int32)
+        t = np.arange(ns)
+        w = sum(np.sin(2 * np.pi * (f * t[None] + r.random((npairs, 1)))) for f in (0.31, 0.37, 0.43))
+        pair = np.repeat(np.arange(npairs), nnear + 1 + nfar)
+        self.samples = (w[pair] + 0.05 * r.standard_normal((n, ns))).astype(np.float32)
+        self.end = end
+        self.params = dict(a0=-1e-4, a1=1e-4, na=5, b0=-9e-8, b1=9e-8, nb=21, c0=0.95e-6, c1=1.05e-6, nc=9, aph=1000,
+                           apm=50, tau=0.0021, azimuth=0.0)
+
+    def arrays(self):
+        z = np.zeros(len(self.sx), np.int32)
+        return semb.GatherArrays(self.end, self.ns, 2000, self.gx, z, self.sx, z, z + 1, self.samples)
+
+
+@pytest.mark.parametrize("form", ["plain", "f32", "f16"])
+@pytest.mark.parametrize("seed,spread", [(0, 0), (1, 0), (2, 1), (3, 2)])
+def test_wide_runs_at_the_record_s_end(seed, spread, form):
+    s = _Scattered(seed, spread=spread)
+    with semb.Plan(semb.params(semb.CRS, **_kw(form), **s.params)) as p:
+        p.set_filter(semb.FILTER_ON)
+        p.upload(s.arrays().view())
+        assert p.filter_tasks()[0] > 0
+        got = _results(p, form)
+        p.set_filter(semb.FILTER_OFF)
+        ref = _results(p, form)
+    for x, y in zip(got, ref):
+        assert np.array_equal(x, y), np.mean(x != y)
+
+
 @pytest.mark.parametrize("variant", [10, 13, 14, 28, 30, 31, 32, 33])
 def test_every_filtered_variant(variant):
     s = _survey(21, 1)
