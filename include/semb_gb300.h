@@ -381,6 +381,11 @@ int semb_probe_fp32(int32_t device, double* tflops);
  * SEMB_E_TIMEOUT instead of a hung GPU, exercised without a fault. */
 int semb_selftest_wait(int32_t device, int64_t limit_us, int32_t* timed_out);
 
+/* Diagnostic with no counterpart in the reference: the square root of the plain search
+ * and CRS-DE on every float of its range, [2^-45, 2^30], in both halves of a pair, against
+ * the correctly rounded root.  *tested gets the number of roots, *wrong those that differ. */
+int semb_selftest_sqrt(int32_t device, int64_t* tested, int64_t* wrong);
+
 /* Number of visible CUDA devices (0 when none); never fails. */
 int32_t semb_device_count(void);
 

@@ -9,8 +9,8 @@
 //   * Items two at a time.  A thread's candidates are pairs, and every operation of a pair
 //     is one FP32x2 instruction (mul, add and FMA round each half as the scalar
 //     instruction does).  Window samples come as scalar loads straight into the halves.
-//   * The square root.  sqrt.rn compiles to a test and a call path around its iteration;
-//     here it is written out for the range that traveltimes have (sqrt2_rn).
+//   * The square root.  Two correctly rounded roots at a time, by Markstein's method, for
+//     the range that squared traveltimes have (sqrt2_rn).
 //   * No range checks where the planner has shown that every item is in range (nearly all
 //     traces); the others take the checked path, in aperture order with them.
 //
@@ -37,10 +37,12 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b, float nz) {
   return __ffma2_rn(a, b, make_float2(nz, nz));
 }
 
-// The correctly rounded square roots of two floats in [2^-45, 2^30]: g = x rsqrt(x), one
-// Newton step on the exact residual x - g^2 (Markstein's final step: g and 1 / (2 g) are
-// good to a few ulp, the FMA residual is exact, and the corrected g rounds correctly).
-// Compared with sqrt.rn on every float of that range.
+// The correctly rounded square roots of two floats in [2^-45, 2^30], after P. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res.
+// Dev. 34 (1990): from y near 1 / sqrt(x), g = x y and h = y / 2 approximate sqrt(x) and
+// 1 / (2 sqrt(x)); the FMA gives the residual x - g^2 without error, and g + h (x - g^2) is
+// so close to sqrt(x) that its one rounding is the root's.  semb_selftest_sqrt compares it
+// with __fsqrt_rn on every float of that range.
 __device__ __forceinline__ float2 sqrt2_rn(float2 x, float nz) {
   const float2 y = make_float2(rsqrt_fast(x.x), rsqrt_fast(x.y));
   const float2 g = mul2(x, y, nz);

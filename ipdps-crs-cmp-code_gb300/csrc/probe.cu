@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include "common.h"
+#include "plain_kernel.cuh"
 #include "semb_kernels.cuh"
 
 namespace {
@@ -94,5 +95,46 @@ extern "C" int semb_selftest_wait(int32_t device, int64_t limit_us, int32_t* tim
   cudaFree(d);
   SEMB_CUDA(e);
   *timed_out = h;
+  return SEMB_OK;
+}
+
+namespace {
+
+// The bit patterns of 2^-45 and 2^30, the range of sqrt2_rn.
+constexpr uint32_t kSqrtLo = (127u - 45u) << 23, kSqrtHi = (127u + 30u) << 23;
+
+// Floats of [2^-45, 2^30] whose sqrt2_rn is not __fsqrt_rn's, in either half of a pair (the
+// other half holds the range backwards).
+__global__ void __launch_bounds__(256) k_sqrt_selftest(float nz, unsigned long long* wrong) {
+  unsigned n = 0;
+  for (uint32_t b = kSqrtLo + blockIdx.x * blockDim.x + threadIdx.x; b <= kSqrtHi; b += gridDim.x * blockDim.x) {
+    const float2 x = make_float2(__uint_as_float(b), __uint_as_float(kSqrtHi - (b - kSqrtLo)));
+    const float2 g = semb::sqrt2_rn(x, nz);
+    n += (__float_as_uint(g.x) != __float_as_uint(__fsqrt_rn(x.x))) +
+         (__float_as_uint(g.y) != __float_as_uint(__fsqrt_rn(x.y)));
+  }
+  if (n) atomicAdd(wrong, (unsigned long long)n);
+}
+
+}  // namespace
+
+extern "C" int semb_selftest_sqrt(int32_t device, int64_t* tested, int64_t* wrong) {
+  if (!tested || !wrong) return semb::fail(SEMB_E_ARG, "null argument");
+  *tested = *wrong = 0;
+  if (device < 0 || device >= semb_device_count()) return semb::fail(SEMB_E_NODEV, "device %d not available", device);
+  SEMB_CUDA(cudaSetDevice(device));
+  unsigned long long* d = nullptr;
+  SEMB_CUDA(cudaMalloc(&d, sizeof(*d)));
+  unsigned long long h = 0;
+  cudaError_t e = cudaMemset(d, 0, sizeof(*d));
+  if (e == cudaSuccess) {
+    k_sqrt_selftest<<<4096, 256>>>(-0.0f, d);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  SEMB_CUDA(e);
+  *tested = 2 * ((int64_t)kSqrtHi - kSqrtLo + 1);
+  *wrong = (int64_t)h;
   return SEMB_OK;
 }

@@ -46,7 +46,8 @@ EXPORTS = [
     "semb_plan_autotune", "semb_plan_buckets", "semb_plan_set_variant", "semb_plan_set_staging",
     "semb_plan_set_filter", "semb_plan_filter_tasks", "semb_plan_set_chunks", "semb_plan_chunk_times",
     "semb_plan_use_graph", "semb_plan_destroy",
-    "semb_host_alloc", "semb_host_free", "semb_probe_fp32", "semb_selftest_wait", "semb_device_count",
+    "semb_host_alloc", "semb_host_free", "semb_probe_fp32", "semb_selftest_wait", "semb_selftest_sqrt",
+    "semb_device_count",
     "semb_strerror", "semb_last_error", "semb_abi_version",
 ]
 
@@ -138,6 +139,7 @@ def lib():
         "semb_host_free": (C.c_int, [P]),
         "semb_probe_fp32": (C.c_int, [i32, P]),
         "semb_selftest_wait": (C.c_int, [i32, i64, P]),
+        "semb_selftest_sqrt": (C.c_int, [i32, P, P]),
         "semb_device_count": (i32, []),
         "semb_strerror": (C.c_char_p, [C.c_int]),
         "semb_last_error": (C.c_char_p, []),
@@ -467,6 +469,14 @@ def selftest_wait(device: int = 0, limit_us: int = 20000) -> int:
     v = C.c_int32()
     _check(lib().semb_selftest_wait(int(device), int(limit_us), C.byref(v)), "semb_selftest_wait")
     return int(v.value)
+
+
+def selftest_sqrt(device: int = 0):
+    """(square roots compared, those that are not correctly rounded) of the plain search's own
+    square root over its whole range."""
+    n, bad = C.c_int64(), C.c_int64()
+    _check(lib().semb_selftest_sqrt(int(device), C.byref(n), C.byref(bad)), "semb_selftest_sqrt")
+    return int(n.value), int(bad.value)
 
 
 def device_count() -> int:
