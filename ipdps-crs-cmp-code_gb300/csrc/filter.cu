@@ -72,10 +72,12 @@ size_t filter_smem(int form, int storage, int nt, int cap) {
   return filter_layout(cap, form == FORM_PLAIN || storage == STORE_F32, form == FORM_PLAIN ? 1 : kTopK, nt).total;
 }
 
-// Whether the direct configuration (window, layout) has a filter and refine pair.
-bool filter_exists(int form, int w, int brun, int pipe, int lay) {
+// Whether the direct configuration (window, layout) has a filter and refine pair.  Not with
+// the global-memory path: a window longer than its stage comes from the FP32 store and ends
+// no chunk, and the refine knows neither.
+bool filter_exists(int form, int w, int brun, int pipe, int lay, int glob) {
   if (form == FORM_PLAIN) return w == 1 || w == 3 || w == 5;
-  return pipe && brun && ((w == 3 && (lay == LAY_PD || lay == LAY_P2)) || (w == 5 && lay == LAY_P2));
+  return pipe && brun && !glob && ((w == 3 && (lay == LAY_PD || lay == LAY_P2)) || (w == 5 && lay == LAY_P2));
 }
 
 // Once per plan configuration, before its launches (which may be captured).

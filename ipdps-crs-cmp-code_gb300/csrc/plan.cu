@@ -53,7 +53,7 @@ constexpr int kMinStage = 512;
 int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, float c, float* out, cudaStream_t st);
 int launch_repick(int w, RepickParams R, int sms, cudaStream_t st);
 int launch_crs_de(int w, const DeParams& R, KParams P, cudaStream_t st);
-bool filter_exists(int form, int w, int brun, int pipe, int lay);
+bool filter_exists(int form, int w, int brun, int pipe, int lay, int glob);
 int filter_shape(int w, int nb, int* rc, int* nt);
 size_t filter_smem(int form, int storage, int nt, int cap);
 int filter_prepare(int form, int w, int storage, int shape);
@@ -465,11 +465,11 @@ float4 sample_candidate(const semb_plan* pl, int gi, bool pad) {
 
 // Put the filter in front of the direct configuration c (variant v) where it pays.
 // SEMB_OK with c.filter null: every candidate is evaluated directly.
-int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int z0, int rc_direct, KernelCfg& c) {
+int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int glob, int z0, int rc_direct, KernelCfg& c) {
   const semb_params& p = pl->p;
   const int form = p.mode == SEMB_PLAIN_F32 ? FORM_PLAIN : FORM_FAST;
   if (pl->filter_mode == SEMB_FILTER_OFF || p.method != SEMB_CRS || p.ngen > 0 || p.nb < 2 ||
-      !filter_exists(form, pl->w, brun, pipe, lay))
+      !filter_exists(form, pl->w, brun, pipe, lay, glob))
     return SEMB_OK;
   int rc = 0, nt = 0;
   const int shape = filter_shape(pl->w, p.nb, &rc, &nt), cs = (rc - 1) / 2;
@@ -729,7 +729,7 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
   c.smem = smem;
   c.occ = occ;
   c.queue = form == FORM_FAST || pipe == 3;
-  const int frc = attach_filter(pl, brun, pipe, lay, z0, rc, c);
+  const int frc = attach_filter(pl, brun, pipe, lay, glob, z0, rc, c);
   if (frc != SEMB_OK) {
     free_cfg(c);
     return frc;

@@ -168,6 +168,29 @@ def test_every_filtered_variant(variant):
     _compare(s, "f16", variant=variant)
 
 
+@pytest.mark.parametrize("tau,variant", [(1, 16), (1, 17), (1, 18), (2, 16)])
+@pytest.mark.parametrize("form", ["f16", "f32"])
+def test_variants_that_do_not_stage_whole_windows_have_no_filter(form, tau, variant):
+    """Their long windows come from the FP32 store and end no chunk, which the refine does not
+    repeat: forced, they evaluate every candidate."""
+    s = synth.crs_survey(seed=72, ncdp=8, noffsets=24, ns=1500, dt_us=4000, na=1, nb=21, nc=5,
+                         tau=tau * 0.004 * 1.0001, aph=2600, apm=50)
+    s.params["c1"] *= 30.0   # a pass spans hundreds of samples
+    arr = _arrays(s)
+    with semb.Plan(semb.params(semb.CRS, **_kw(form), **s.params)) as p:
+        p.set_filter(semb.FILTER_ON)
+        p.upload(arr.view())
+        p.set_staging(128)
+        assert p.filter_tasks()[0] > 0
+        p.set_variant(variant)
+        got = _results(p, form)
+        assert p.filter_tasks() == (0, 0)
+        p.set_filter(semb.FILTER_OFF)
+        ref = _results(p, form)
+    for x, y in zip(got, ref):
+        assert np.array_equal(x, y), (np.mean(x != y), np.abs(x - y).max())
+
+
 @pytest.mark.parametrize("form", ["plain", "f16", "bf16", "f32"])
 def test_apertures_of_one_cdp_overflow_into_the_direct_kernel(form):
     """Every A and B ties: no list holds them all."""
