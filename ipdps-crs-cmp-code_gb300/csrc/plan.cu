@@ -160,6 +160,7 @@ struct semb_plan {
   int2* d_fb_tasks = nullptr;
   int* d_fb_count = nullptr;
   int filter_mode = SEMB_FILTER_AUTO;
+  double moved = 1.0;   // CRS: share of the aperture traces whose CDPs tell the values of A apart
   int* d_status = nullptr;
   unsigned long long* d_repicked = nullptr;
   // extra attributes (batched form with attrs = 1)
@@ -482,7 +483,13 @@ int attach_filter(semb_plan* pl, int brun, int pipe, int lay, int glob, int z0, 
   // 7 x 21 x 7 grid with little more than one task per SM 1.5 and 1.3.
   const double direct = (form == FORM_PLAIN ? 73.0 : 25.0 + (pl->w == 5 ? 8.0 : 0.0)) * (double)pl->ncand;
   const double filtered = (100.0 + 3.5 * rc) * (double)total + (form == FORM_PLAIN ? 3500.0 : 8600.0);
-  if (filtered > 0.9 * direct && pl->filter_mode != SEMB_FILTER_ON) return SEMB_OK;
+  // A CDP on which no traveltime depends on A (apertures of one CDP, whose midpoints agree)
+  // takes both: its lists overflow.  200 CDPs of the line with an aperture of 5 m took 75.2 ms
+  // so in the batched form and 68.0 without the filter (w = 5: 115.0 and 105.1); in the plain
+  // form, whose candidates cost three times as much, what does not overflow still pays (40 CDPs
+  // 26.8 and 28.9).
+  const double share = form == FORM_PLAIN ? 0.9 : pl->moved - 0.1;
+  if (filtered > share * direct && pl->filter_mode != SEMB_FILTER_ON) return SEMB_OK;
   // each (A, C) group's B values cut into the fewest runs of at most rc, of equal length
   // give or take one, each run's middle value in slot cs, B ascending with the slot; padding
   // repeats the run's ends
@@ -1095,12 +1102,17 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
   // azimuth direction for the signed midpoint displacement (SEMB_DM_SIGNED)
   const double az = p.azimuth * 3.14159265358979323846 / 180.0;
   const double cos_d = std::cos(az), sin_d = std::sin(az);
+  // the share of the aperture traces whose CDPs tell the values of A apart: A's range moves
+  // some traveltime by 0.01 samples (counted in d_repicked, which every run resets)
+  const double a_range = std::fabs(p.a1 - p.a0) * pl->idt64;
+  const float m_min = p.method == SEMB_CRS && p.na > 1 ? (float)(0.01 / a_range) : -1.f;
+  SEMB_CUDA(cudaMemsetAsync(pl->d_repicked, 0, sizeof(unsigned long long), st));
   k_aperture_fill<<<(g->ncdps + 7) / 8, 256, 0, st>>>(g->ncdps, p.method, pl->d_nbr_off, pl->d_nbr, d_cdp_end,
                                                        pl->d_ap_off, d_h32, d_mx32, d_my32, d_h64, d_mx64, d_my64,
                                                        pl->d_ap_tr, pl->d_ap_geo, pl->d_ap_geo64,
                                                        ff ? pl->d_ap_ff : nullptr,
                                                        p.dm_mode == SEMB_DM_SIGNED ? 1 : 0, (float)cos_d,
-                                                       (float)sin_d, cos_d, sin_d);
+                                                       (float)sin_d, cos_d, sin_d, m_min, pl->d_repicked);
   SEMB_CUDA(cudaGetLastError());
   if (p.method == SEMB_CRS) {
     SEMB_TRY(dev_reuse(pl, &pl->d_z0r, g->ncdps));
@@ -1140,7 +1152,10 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
     for (int ic = 0; ic < p.nc; ++ic) cv[ic] = (float)(pl->g64[3 * (size_t)ic + 2] * (pl->idt64 * pl->idt64));
     SEMB_TRY(dev_reuse(pl, &pl->d_cvals, cv.size()));
     SEMB_CUDA(cudaMemcpyAsync(pl->d_cvals, cv.data(), cv.size() * 4, cudaMemcpyHostToDevice, st));
+    unsigned long long moved = 0;
+    SEMB_CUDA(cudaMemcpyAsync(&moved, pl->d_repicked, sizeof(moved), cudaMemcpyDeviceToHost, st));
     SEMB_CUDA(cudaStreamSynchronize(st));   // cv is a host temporary
+    pl->moved = (double)moved / (double)std::max<int64_t>(pl->nap, 1);
   }
 
   // work queue: (cdp, t0 block), largest aperture first (longest-processing-time order)
@@ -1514,7 +1529,8 @@ int enqueue_repick(semb_plan* pl, cudaStream_t st, int cdp0, int cdp1, bool rese
     R.ap_off = pl->d_ap_off;
     R.ap_tr = pl->d_ap_tr;
     R.ap_geo64 = pl->d_ap_geo64;
-    R.ap_ff = p.attrs ? nullptr : pl->d_ap_ff;
+    // where no traveltime depends on A its values tie exactly, which only FP64 settles
+    R.ap_ff = p.attrs || pl->moved < 0.5 ? nullptr : pl->d_ap_ff;
     R.cand64 = pl->d_cand64;
     R.stt00 = pl->d_stt00;
     R.ncdps = pl->ncdps;

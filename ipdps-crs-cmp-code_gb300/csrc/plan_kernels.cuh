@@ -167,7 +167,8 @@ __device__ __forceinline__ void store_pairs(float4* out, const Geo64& g) {
 // first trace (CRS/OpenMP/src/main.cpp:179-204, 289-317), in float and in double.
 // With `signed_dm` (SEMB_DM_SIGNED, no reference counterpart) dm is the midpoint
 // displacement projected on the azimuth direction (cos, sin), signed, and dm^2 its
-// square.  CMP apertures are the CDP's own traces with dm = 0.
+// square.  CMP apertures are the CDP's own traces with dm = 0.  *moved gains the aperture
+// traces of the CDPs on which some |dm| exceeds m_min.
 static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __restrict__ nbr_off,
                                 const int32_t* __restrict__ nbr, const int64_t* __restrict__ cdp_end,
                                 const int64_t* __restrict__ ap_off, const float* __restrict__ h32,
@@ -176,7 +177,8 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
                                 const double* __restrict__ my64, int32_t* __restrict__ ap_tr,
                                 float4* __restrict__ ap_geo, Geo64* __restrict__ ap_geo64,
                                 float4* __restrict__ ap_ff, int signed_dm,
-                                float cos_f, float sin_f, double cos_d, double sin_d) {
+                                float cos_f, float sin_f, double cos_d, double sin_d, float m_min,
+                                unsigned long long* __restrict__ moved) {
   const int warps = blockDim.x >> 5;
   const int i = blockIdx.x * warps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -185,15 +187,17 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
   const float cx = mx32[first], cy = my32[first];
   const double cxd = mx64[first], cyd = my64[first];
   int64_t pos = ap_off[i];
+  bool moves = false;
   for (int64_t q = nbr_off[i]; q < nbr_off[i + 1]; ++q) {
     const int j = nbr[q];
     const int64_t t0 = j > 0 ? cdp_end[j - 1] : 0, t1 = cdp_end[j];
     for (int64_t t = t0 + lane; t < t1; t += 32) {
       const int64_t e = pos + (t - t0);
       ap_tr[e] = (int32_t)t;
+      float m = 0.f;
       if (method == METHOD_CRS && signed_dm) {
         const float dx = __fsub_rn(mx32[t], cx), dy = __fsub_rn(my32[t], cy);
-        const float m = __fadd_rn(__fmul_rn(dx, cos_f), __fmul_rn(dy, sin_f));
+        m = __fadd_rn(__fmul_rn(dx, cos_f), __fmul_rn(dy, sin_f));
         ap_geo[e] = make_float4(m, __fmul_rn(m, m), h32[t], 0.f);
         const double dxd = __dsub_rn(mx64[t], cxd), dyd = __dsub_rn(my64[t], cyd);
         const double md = __dadd_rn(__dmul_rn(dxd, cos_d), __dmul_rn(dyd, sin_d));
@@ -203,7 +207,8 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
       } else if (method == METHOD_CRS) {
         const float dx = __fsub_rn(mx32[t], cx), dy = __fsub_rn(my32[t], cy);
         const float m2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-        ap_geo[e] = make_float4(__fsqrt_rn(m2), m2, h32[t], 0.f);
+        m = __fsqrt_rn(m2);
+        ap_geo[e] = make_float4(m, m2, h32[t], 0.f);
         const double dxd = __dsub_rn(mx64[t], cxd), dyd = __dsub_rn(my64[t], cyd);
         const double m2d = __dadd_rn(__dmul_rn(dxd, dxd), __dmul_rn(dyd, dyd));
         const Geo64 g = {__dsqrt_rn(m2d), m2d, h64[t], 0.0};
@@ -213,9 +218,12 @@ static __global__ void k_aperture_fill(int ncdps, int method, const int64_t* __r
         ap_geo[e] = make_float4(0.f, 0.f, h32[t], 0.f);
         ap_geo64[e] = Geo64{0.0, 0.0, h64[t], 0.0};
       }
+      moves = moves || fabsf(m) > m_min;
     }
     pos += t1 - t0;
   }
+  moves = __any_sync(0xffffffffu, moves);
+  if (lane == 0 && moves) atomicAdd(moved, (unsigned long long)(pos - ap_off[i]));
 }
 
 // CRS: where each CDP's own traces sit in its aperture list (k_aperture_fill appends

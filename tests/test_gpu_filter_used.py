@@ -250,15 +250,23 @@ def test_streamed_chunked_and_graph_runs(form, tau):
 @pytest.mark.parametrize("form", ["plain", "f16"])
 def test_default_use(form):
     """Where it pays: the 21 x 21 x 21 grid, not a 3 x 3 x 3 one or one B value, never CMP."""
-    def tasks(**kw):
+    def tasks(signed=False, azimuth=0.0, **kw):
         s = _survey(ns=600, tau=1, ncdp=3, **kw)
-        with semb.Plan(semb.params(semb.CRS, **_kw(form), **s.params)) as p:
+        s.params["azimuth"] = azimuth
+        with semb.Plan(semb.params(semb.CRS, **_kw(form, signed), **s.params)) as p:
             p.upload(_arrays(s).view())
             return p.filter_tasks()[0]
 
     assert tasks(na=21, nb=21, nc=21) > 0
     assert tasks(na=3, nb=3, nc=3) == 0
     assert tasks(na=21, nb=1, nc=21) == 0
+    # apertures in which no traveltime depends on A (batched form): one CDP; a line across the
+    # azimuth
+    pays = form == "plain"
+    assert (tasks(na=21, nb=21, nc=21, apm=5) > 0) == pays
+    assert (tasks(na=21, nb=21, nc=21, azimuth=90.0, signed=True) > 0) == pays
+    assert tasks(na=21, nb=21, nc=21, azimuth=30.0, signed=True) > 0
+    assert tasks(na=1, nb=21, nc=441, apm=5) > 0
     s = synth.cmp_survey(seed=1, ncmp=2, half_offsets=np.linspace(10.0, 300.0, 20), ns=320, nc=64, tau=0.0021)
     g = oracle.gather(s.headers, s.samples, "cmp", s.params["aph"])
     arr = semb.GatherArrays(g["ntraces_by_cdp_id"], g["ns"], g["dt_us"], g["gx"], g["gy"], g["sx"], g["sy"],
