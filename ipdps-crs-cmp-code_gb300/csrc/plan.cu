@@ -244,16 +244,19 @@ void dev_free(T*& p) {
   p = nullptr;
 }
 
+void free_filter(KernelCfg& c) {
+  if (!c.filter) return;
+  dev_free(c.filter->d_cand);
+  dev_free(c.filter->d_pass_bounds);
+  delete c.filter;
+  c.filter = nullptr;
+}
+
 void free_cfg(KernelCfg& c) {
   dev_free(c.d_cand);
   dev_free(c.d_pass_bounds);
   dev_free(c.d_pass_c);
-  if (c.filter) {
-    dev_free(c.filter->d_cand);
-    dev_free(c.filter->d_pass_bounds);
-    delete c.filter;
-    c.filter = nullptr;
-  }
+  free_filter(c);
   c.variant = -1;
 }
 
@@ -273,20 +276,38 @@ void dev_release(semb_plan* pl, T*& p) {
 }
 
 // Gives back the buffers that a plan can do without (the re-pick's paired geometry and the
-// filter's lists); false where there are none.
+// filter's lists), with the filters and the captured launches that hold them; false where
+// there are none.
 bool drop_optional(semb_plan* pl) {
   const bool any = pl->d_ap_ff || pl->d_head || pl->d_pool || pl->d_fb_tasks;
+  if (!any) return false;
+  for (Bucket& b : pl->buckets) free_filter(b.cfg);
+  if (pl->graph) cudaGraphExecDestroy(pl->graph);
+  pl->graph = nullptr;
+  for (auto& c : pl->run_chunks) {
+    if (c.graph) cudaGraphExecDestroy(c.graph);
+    c.graph = nullptr;
+  }
   dev_release(pl, pl->d_ap_ff);
   dev_release(pl, pl->d_head);
   dev_release(pl, pl->d_pool);
   dev_release(pl, pl->d_fb_tasks);
-  return any;
+  return true;
+}
+
+// dev_alloc of something a plan needs: out of memory, the optional buffers go before it fails.
+template <typename T>
+int dev_need(semb_plan* pl, T** p, size_t n) {
+  int rc = dev_alloc(p, n);
+  if (rc == SEMB_E_NOMEM) {
+    cudaGetLastError();
+    if (drop_optional(pl)) rc = dev_alloc(p, n);
+  }
+  return rc;
 }
 
 // Device buffer *p of n elements, kept from the previous upload when it is large
-// enough (re-uploads of a survey of the same size then allocate nothing).  An upload that
-// runs out of memory gives the optional buffers back before it fails (no launch
-// configuration holds them then).
+// enough (re-uploads of a survey of the same size then allocate nothing).
 template <typename T>
 int dev_reuse(semb_plan* pl, T** p, size_t n, bool optional = false) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
@@ -295,12 +316,11 @@ int dev_reuse(semb_plan* pl, T** p, size_t n, bool optional = false) {
   if (*p) cudaFree(*p);
   *p = nullptr;
   pl->caps.erase(p);
-  int rc = dev_alloc(p, n);
-  if (rc == SEMB_E_NOMEM) {
+  const int rc = optional ? dev_alloc(p, n) : dev_need(pl, p, n);
+  if (rc != SEMB_OK) {
     cudaGetLastError();
-    if (!optional && !pl->uploaded && drop_optional(pl)) rc = dev_alloc(p, n);
+    return rc;
   }
-  if (rc != SEMB_OK) return rc;
   pl->caps[p] = bytes;
   return SEMB_OK;
 }
@@ -711,8 +731,8 @@ int build_cfg(semb_plan* pl, int v, KernelCfg& out) {
     widen_bounds(pl, &bounds[(size_t)(k / cpp) * 8], k % cpp == 0, gi);
   }
   KernelCfg c;
-  if (dev_alloc(&c.d_cand, npad) != SEMB_OK || dev_alloc(&c.d_pass_bounds, bounds.size()) != SEMB_OK ||
-      (z0 && dev_alloc(&c.d_pass_c, pass_c.size()) != SEMB_OK)) {
+  if (dev_need(pl, &c.d_cand, npad) != SEMB_OK || dev_need(pl, &c.d_pass_bounds, bounds.size()) != SEMB_OK ||
+      (z0 && dev_need(pl, &c.d_pass_c, pass_c.size()) != SEMB_OK)) {
     free_cfg(c);
     return fail(SEMB_E_NOMEM, "candidate table of %d entries", npad);
   }
@@ -1060,14 +1080,20 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
     k_cdp_midpoints<<<nc_blocks, 256, 0, st>>>(g->ncdps, d_cdp_end, d_gx, d_gy, d_sx, d_sy, d_sc, d_fmx, d_fmy);
     if (g->ncdps >= kGridNeighbours) {
       // large surveys: grid cells + sorts, O(n log n); the same lists
-      SEMB_TRY(grid_neighbours(g->ncdps, d_fmx, d_fmy, p.apm, pl->d_nbr_off, &pl->d_nbr, &pl->n_nbr, st));
+      auto lists = [&] { return grid_neighbours(g->ncdps, d_fmx, d_fmy, p.apm, pl->d_nbr_off, &pl->d_nbr, &pl->n_nbr, st); };
+      int rc = lists();
+      if (rc == SEMB_E_NOMEM) {
+        cudaGetLastError();
+        if (drop_optional(pl)) rc = lists();
+      }
+      SEMB_TRY(rc);
     } else {
       const float lim = (float)((int32_t)p.apm * (int32_t)p.apm);
       k_neighbours<<<nc_blocks, 256, 0, st>>>(g->ncdps, d_fmx, d_fmy, lim, d_cnt32, nullptr, nullptr);
       k_scan_exclusive<int32_t><<<1, 1024, 0, st>>>(g->ncdps, d_cnt32, pl->d_nbr_off);
       SEMB_CUDA(cudaMemcpyAsync(&pl->n_nbr, pl->d_nbr_off + g->ncdps, 8, cudaMemcpyDeviceToHost, st));
       SEMB_CUDA(cudaStreamSynchronize(st));
-      SEMB_TRY(dev_alloc(&pl->d_nbr, (size_t)pl->n_nbr));
+      SEMB_TRY(dev_need(pl, &pl->d_nbr, (size_t)pl->n_nbr));
       k_neighbours<<<nc_blocks, 256, 0, st>>>(g->ncdps, d_fmx, d_fmy, lim, nullptr, pl->d_nbr_off, pl->d_nbr);
     }
   } else {
@@ -1254,9 +1280,9 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
     SEMB_TRY(dev_reuse(pl, &pl->d_top_idx, nout * kTopK));
     SEMB_TRY(dev_reuse(pl, &pl->d_top_stk, nout * kTopK));
     if (p.attrs) {
-      SEMB_TRY(dev_alloc(&pl->d_sem2, nout));
-      SEMB_TRY(dev_alloc(&pl->d_idx2, nout));
-      SEMB_TRY(dev_alloc(&pl->d_err64, nout));
+      SEMB_TRY(dev_need(pl, &pl->d_sem2, nout));
+      SEMB_TRY(dev_need(pl, &pl->d_idx2, nout));
+      SEMB_TRY(dev_need(pl, &pl->d_err64, nout));
     }
   }
   if (p.ngen > 0) {
@@ -1266,7 +1292,7 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
       grid[3 * (size_t)i + 1] = pl->gb[i];
       grid[3 * (size_t)i + 2] = pl->gc[i];
     }
-    SEMB_TRY(dev_alloc(&pl->d_grid, grid.size()));
+    SEMB_TRY(dev_need(pl, &pl->d_grid, grid.size()));
     SEMB_CUDA(cudaMemcpyAsync(pl->d_grid, grid.data(), grid.size() * 4, cudaMemcpyHostToDevice, st));
     SEMB_CUDA(cudaStreamSynchronize(st));
     const float lo[3] = {(float)p.a0, (float)p.b0, (float)(p.c0 * kFactor)};
@@ -1276,11 +1302,11 @@ int upload_impl(semb_plan* pl, const semb_gather_view* g, int nchunks) {
       box[2 * d] = std::min(lo[d], hi[d]);
       box[2 * d + 1] = std::max(lo[d], hi[d]);
     }
-    SEMB_TRY(dev_alloc(&pl->d_de_box, 8));
+    SEMB_TRY(dev_need(pl, &pl->d_de_box, 8));
     SEMB_CUDA(cudaMemcpy(pl->d_de_box, box, sizeof(box), cudaMemcpyHostToDevice));
-    SEMB_TRY(dev_alloc(&pl->d_de_a, nout));
-    SEMB_TRY(dev_alloc(&pl->d_de_b, nout));
-    SEMB_TRY(dev_alloc(&pl->d_de_c, nout));
+    SEMB_TRY(dev_need(pl, &pl->d_de_a, nout));
+    SEMB_TRY(dev_need(pl, &pl->d_de_b, nout));
+    SEMB_TRY(dev_need(pl, &pl->d_de_c, nout));
   }
   pl->aperture.resize(g->ncdps);
   for (int i = 0; i < g->ncdps; ++i) pl->aperture[i] = (int32_t)(ap_off[i + 1] - ap_off[i]);
@@ -1661,7 +1687,7 @@ int build_run_chunks(semb_plan* pl) {
     if (q != cdps.size()) return fail(SEMB_E_STATE, "aperture buckets do not cover chunk %d", (int)pl->run_chunks.size());
     pl->run_chunks.push_back(std::move(ch));
   }
-  SEMB_TRY(dev_alloc(&pl->d_chunk_tasks, tasks.size()));
+  SEMB_TRY(dev_need(pl, &pl->d_chunk_tasks, tasks.size()));
   SEMB_CUDA(cudaMemcpy(pl->d_chunk_tasks, tasks.data(), tasks.size() * sizeof(int2), cudaMemcpyHostToDevice));
   const size_t nev = pl->run_chunks.size() + 1;
   while (pl->chunk_ev.size() < nev) {
@@ -1956,7 +1982,7 @@ int semb_plan_autotune(semb_plan* pl, int32_t* chosen, double* ms_of_variant) {
   SEMB_CUDA(cudaMemcpy(all.data(), pl->d_tasks, all.size() * sizeof(int2), cudaMemcpyDeviceToHost));
   const int smax = std::max(1, pl->sms * 8);
   int2* d_sample = nullptr;
-  SEMB_TRY(dev_alloc(&d_sample, smax));
+  SEMB_TRY(dev_need(pl, &d_sample, smax));
   struct Free {
     int2* p;
     KernelCfg trial;
