@@ -160,10 +160,14 @@ __global__ void __launch_bounds__(kDeWarps * 32, 2) k_crs_de(DeParams R, KParams
       const ChunkMeta* meta = meta_at(cur);
       bool ok = true;
       if (!ready) {
-        ok = wait_bar(&full[cur], (phases >> cur) & 1u);
+        const uint32_t parity = (phases >> cur) & 1u;
+        ok = wait_bar(&full[cur], parity);
         phases ^= 1u << cur;
         if (__syncthreads_or(!ok)) {
           if (threadIdx.x == 0) atomicOr(P.status, ST_TIMEOUT);
+          // the late copy still writes this CTA's shared memory: wait for it (bounded); the
+          // other buffer has none under way
+          wait_bar(&full[cur], parity);
           return false;
         }
       }
