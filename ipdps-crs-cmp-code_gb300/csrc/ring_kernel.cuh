@@ -11,13 +11,23 @@
 // What bounds it: latency and the FP32 pipe together (w = 5: 25 FP32 operations per
 // trace-evaluation on 33 cycles).  256 CMPs of the uneven-fold line (256 velocities, w = 5)
 // 10.29 ms in the two-barrier kernel (79% of the shared-memory pipe for its 16-byte entries),
-// 9.34 here; w = 11, 90 velocities 0.57 -> 0.46.  The trace loop unrolled by two: 1 to 2%.
+// 9.45 here; w = 11, 90 velocities 0.57 -> 0.46.  The trace loop unrolled by two: 1 to 2%.
 // ring_variant() (launch.cu) says where it is used and has both sides.
 #pragma once
 
 #include "filter_kernel.cuh"
 
 namespace semb {
+
+// Traces whose energy one FP32 chain sums before it is folded into the Kahan total (almost
+// twice as many where a chunk's last in-range traces and the others meet).  A chunk holds up
+// to 128; the two-barrier kernel's entries leave room for some 60, in two chains up to w = 5.
+// In one chain per chunk the semblance's rms distance from 64 bits was above that kernel's
+// with the FP32 store: w = 7, fold 200 2.70e-7 against 2.67e-7 in chains of 64, 2.81e-7 in
+// whole chunks, 2.63e-7 so.  It costs 1.4% on the uneven-fold line (9.32 -> 9.45 ms), up to 5%
+// with 10 candidates per thread; one copy of the fold for all traces 3.3% and 2%, chunks of
+// 32 traces 7%.
+constexpr int kRingFold = 32;
 
 // Shared-memory layout (bytes), shared by host and device:
 //   [0, 128)   mbarriers (full[3], q_full[3], q_empty[3], merge_done) and the merge counter
@@ -275,28 +285,46 @@ __global__ void __launch_bounds__(NT, 1) semb_ring_kernel(KParams P) {
         s0 = s1;
       }
     };
-#pragma unroll 2
-    for (int e = 0; e < n_in; ++e) {   // every item in range
-      const float4 g = meta->geo[e];
-      const uint32_t base = plane + 4u * (uint32_t)(__float_as_int(g.w) - P.tau) - 4u * 0x4B000000u;
-      const float2 gz = make_float2(g.z, g.z);
+    // Kahan: fold the energy since the last time into the compensated totals
+    auto fold = [&]() {
 #pragma unroll
-      for (int p = 0; p < RP; ++p) {
-        const float2 q = __ffma2_rn(cc[p], gz, T22);
-        const float2 t = make_float2(sqrt_fast(q.x), sqrt_fast(q.y));
-        const float2 y = __fadd2_rz(t, k23);
-        const float2 x = __ffma2_rn(__fadd2_rn(y, km23), kNeg, t);   // t - floor(t)
-        if constexpr (SEMB_CHECKED) {
-          const int i0 = __float_as_int(g.w) - P.tau - 0x4B000000;
-          report_window(P.status, __float_as_int(y.x) + i0, W, src_at(c)[e], tg.cdp, t0);
-          report_window(P.status, __float_as_int(y.y) + i0, W, src_at(c)[e], tg.cdp, t0);
+      for (int r = 0; r < RC; ++r) {
+        const float hi = kahan_hi[r * NT], lo = kahan_lo[r * NT];
+        const float yv = ((r & 1) ? den[r >> 1].y : den[r >> 1].x) - lo;
+        const float tv = hi + yv;
+        kahan_lo[r * NT] = (tv - hi) - yv;
+        kahan_hi[r * NT] = tv;
+      }
+#pragma unroll
+      for (int p = 0; p < RP; ++p) den[p] = make_float2(0.f, 0.f);
+    };
+    for (int e0 = 0; e0 < n_in; e0 += kRingFold) {   // every item in range
+      if (e0 > 0) fold();
+      const int e1 = min(n_in, e0 + kRingFold);
+#pragma unroll 2
+      for (int e = e0; e < e1; ++e) {
+        const float4 g = meta->geo[e];
+        const uint32_t base = plane + 4u * (uint32_t)(__float_as_int(g.w) - P.tau) - 4u * 0x4B000000u;
+        const float2 gz = make_float2(g.z, g.z);
+#pragma unroll
+        for (int p = 0; p < RP; ++p) {
+          const float2 q = __ffma2_rn(cc[p], gz, T22);
+          const float2 t = make_float2(sqrt_fast(q.x), sqrt_fast(q.y));
+          const float2 y = __fadd2_rz(t, k23);
+          const float2 x = __ffma2_rn(__fadd2_rn(y, km23), kNeg, t);   // t - floor(t)
+          if constexpr (SEMB_CHECKED) {
+            const int i0 = __float_as_int(g.w) - P.tau - 0x4B000000;
+            report_window(P.status, __float_as_int(y.x) + i0, W, src_at(c)[e], tg.cdp, t0);
+            report_window(P.status, __float_as_int(y.y) + i0, W, src_at(c)[e], tg.cdp, t0);
+          }
+          window(p, min(__float_as_uint(y.x) * 4u + base, top), min(__float_as_uint(y.y) * 4u + base, top), x);
         }
-        window(p, min(__float_as_uint(y.x) * 4u + base, top), min(__float_as_uint(y.y) * 4u + base, top), x);
       }
     }
     // the other traces: per-item range checks; an out-of-range item reads the zero block
     // with weight 0 and does not count
     for (int e = kMaxChunk - (n - n_in); e < kMaxChunk; ++e) {
+      if ((kMaxChunk - e) % kRingFold == 0) fold();
       const float4 g = meta->geo[e];
       const int soff = __float_as_int(g.w);
 #pragma unroll
@@ -322,17 +350,7 @@ __global__ void __launch_bounds__(NT, 1) semb_ring_kernel(KParams P) {
     // the plane and metadata of chunk c are no longer read by this warp
     __syncwarp();
     if (lane == 0) mbar_arrive(&q_empty[c % kStages]);
-    // Kahan: fold this chunk's energy into the compensated totals
-#pragma unroll
-    for (int r = 0; r < RC; ++r) {
-      const float hi = kahan_hi[r * NT], lo = kahan_lo[r * NT];
-      const float yv = ((r & 1) ? den[r >> 1].y : den[r >> 1].x) - lo;
-      const float tv = hi + yv;
-      kahan_lo[r * NT] = (tv - hi) - yv;
-      kahan_hi[r * NT] = tv;
-    }
-#pragma unroll
-    for (int p = 0; p < RP; ++p) den[p] = make_float2(0.f, 0.f);
+    fold();
 
     if (tg.flags & CH_PASS_LAST) {
       // ---- finalize the pass's items into this thread's top-4 ----
