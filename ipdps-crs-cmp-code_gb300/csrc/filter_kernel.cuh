@@ -47,9 +47,13 @@
 // s sqrt(sum d_j^2), s = t 2^-24; the filter's own rounding adds as much.  The bounds
 // take `kappa` times that (8 in the batched form; 16 in the plain form, whose
 // traveltimes are rounded more often), growing with sqrt(N) for what may not be random,
-// and a relative 4e-6 and up for the order of the FP32 sums.  Where an energy is all
-// rounding, or not finite, or where rounding decides whether a trace is in the record,
-// the item is kept.
+// and a relative 4e-6 and up for the order of the FP32 sums.  A trace's slopes are the
+// steepest of its run: beyond a boundary that an item crosses, or may cross by its
+// rounding (`edge`), and of every item of a trace that goes on its own.  Where an energy is
+// all rounding, or not finite, or where rounding decides whether a trace is in the record,
+// the item is kept.  The bounds are a multiple of an rms, not a worst case (which, some 8 s
+// sum |d_j|, would keep ten times the candidates): what the filter leaves out has lost
+// unless a rounding lies outside them.
 //
 // Windows are staged as plain FP32 samples (4 bytes each, a chunk holds up to 128
 // traces): straight from the FP32 store by TMA, or, for a 16-bit store, converted once
@@ -417,6 +421,8 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
   const float q_lo = (float)(P.tau * P.tau), q_hi = (float)(P.ns - P.tau - 1) * (float)(P.ns - P.tau - 1);
   const float hdB = 0.5f * P.dB;
   const float sig = (float)P.ns * 5.9604645e-8f;   // t 2^-24 at the record's end
+  // within this of a sample boundary the direct kernel's rounding may lie across it
+  const float edge = 8.f * sig;
   float T = 0.f;
   // the warp's run: A, C and the centre's B; the real slots and their widest offset
   float ca = 0.f, cb = 0.f, cc = 0.f, rmax = 0.f;
@@ -498,7 +504,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
                           tg.cdp, t0);
           }
           ms.template add<QUAD>(a, x, k1, QUAD ? (k1 * k1) * ti : 0.f);
-          const float h = k1 * rmax;
+          const float h = fmaf(k1, rmax, edge);
           if (x + h >= 1.0f) um |= 1u << (e - 32 * b);
           if (x < h) dm |= 1u << (e - 32 * b);
         }
@@ -517,6 +523,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
     for (int e = kMaxChunk - (n - n_in); e < kMaxChunk; ++e) {
       const float4 g = meta->geo[e];
       const int soff = __float_as_int(g.w);
+      float hm = 0.f;   // the most of its items' sums of squared slopes (padding: no less)
       const float u = fmaf(ca, g.x, T);
       const float q0 = fmaf(u, u, cc * g.z);
       const int kind = meta->raw[e];
@@ -540,7 +547,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
             if ((valid >> (2 * pr + 1)) & 1)
               report_window(P.status, __float_as_int(y.y) + i0, W, src_at(c)[e], tg.cdp, t0);
           }
-          float2 s0 = make_float2(lds32(ax), lds32(ay));
+          float2 s0 = make_float2(lds32(ax), lds32(ay)), hs = make_float2(0.f, 0.f);
 #pragma unroll
           for (int j = 0; j < W; ++j) {
             const float2 s1 = make_float2(lds32(ax + 4u * (j + 1)), lds32(ay + 4u * (j + 1)));
@@ -548,10 +555,12 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
             const float2 v = __ffma2_rn(d, x, s0);
             inum[j][pr] = __fadd2_rn(inum[j][pr], v);
             iden[pr] = __ffma2_rn(v, v, iden[pr]);
-            if (pr == CS / 2) ms.h = (CS & 1) ? fmaf(d.y, d.y, ms.h) : fmaf(d.x, d.x, ms.h);
+            hs = __ffma2_rn(d, d, hs);
             s0 = s1;
           }
+          hm = fmaxf(hm, fmaxf(hs.x, hs.y));
         }
+        ms.h += hm;
         continue;
       }
       bool single = true;
@@ -571,7 +580,8 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
           ms.template add<true>(a, in ? x : 0.f, in ? k1 : 0.f, in ? (k1 * k1) * ti : 0.f);
         }
         if (in) {
-          const uint32_t up = x + k1 * rmax >= 1.0f ? 1u << (e & 31) : 0u, dn = x < k1 * rmax ? 1u << (e & 31) : 0u;
+          const float hc = fmaf(k1, rmax, edge);
+          const uint32_t up = x + hc >= 1.0f ? 1u << (e & 31) : 0u, dn = x < hc ? 1u << (e & 31) : 0u;
 #pragma unroll
           for (int b = 0; b < kMaxChunk / 32; ++b)
             if (e >> 5 == b) {
@@ -617,7 +627,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
           }
           const uint32_t ax = okx ? min(plane + 4u * (uint32_t)(soff + relx), top) : top;
           const uint32_t ay = oky ? min(plane + 4u * (uint32_t)(soff + rely), top) : top;
-          float2 s0 = make_float2(lds32(ax), lds32(ay));
+          float2 s0 = make_float2(lds32(ax), lds32(ay)), hs = make_float2(0.f, 0.f);
 #pragma unroll
           for (int j = 0; j < W; ++j) {
             const float2 s1 = make_float2(lds32(ax + 4u * (j + 1)), lds32(ay + 4u * (j + 1)));
@@ -625,10 +635,12 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
             const float2 v = __ffma2_rn(d, x, s0);
             inum[j][pr] = __fadd2_rn(inum[j][pr], v);
             iden[pr] = __ffma2_rn(v, v, iden[pr]);
-            if (pr == CS / 2) ms.h = (CS & 1) ? fmaf(d.y, d.y, ms.h) : fmaf(d.x, d.x, ms.h);
+            hs = __ffma2_rn(d, d, hs);
             s0 = s1;
           }
+          hm = fmaxf(hm, fmaxf(hs.x, hs.y));
         }
+        ms.h += hm;
         if (single) {
           unsure |= near_end;
           miss2 |= miss1 & off_now & ~near_end;
@@ -689,6 +701,9 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
           q1 = fmaf(cj[j], p[j + 1], q1);
           q2 = fmaf(cj[j], fmaf(2.f, UP ? dm : -dp, cj[j]), q2);
         }
+        // the slopes beyond the boundary, where they are the larger ones: q2 is the difference
+        // of the two intervals' sums of squared slopes
+        ms.h += fmaxf(q2, 0.f);
         const float2 z02 = make_float2(z0, z0), a12 = make_float2(a1, a1), a22 = make_float2(a2, a2);
         const float2 q12 = make_float2(2.f * q1, 2.f * q1), q22 = make_float2(q2, q2);
         // only the slots on that side of the centre

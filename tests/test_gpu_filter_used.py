@@ -95,6 +95,48 @@ def test_geometries(case, form, signed, tau):
     _compare(_survey(21, tau, az=30.0 if signed else 0.0, **case), form, signed=signed)
 
 
+def _spikes(r, ns, repeat, ncdp, fold, spacing, noise, early):
+    """Traces of isolated spikes in next to no noise, each geometry `repeat` times: where a
+    traveltime comes near a spike, the next interval's slopes are all that counts."""
+    cdp, off = np.divmod(np.arange(ncdp * fold).repeat(repeat), fold)
+    mx, half = np.round(10 * spacing * cdp).astype(int), r.choice([0, 100, 2000]) + 100 * off
+    n = len(mx)
+    base = np.zeros(ns)
+    base[r.integers(0, ns // 3 if early else ns, 12)] = 1.0
+    amp = 1.0 + 0.3 * r.standard_normal((n, 1))
+    smp = (amp * base + noise * r.standard_normal((n, ns))).astype(np.float32)
+    z = np.zeros(n, np.int32)
+    return semb.GatherArrays((1 + np.arange(ncdp)) * fold * repeat, ns, 4000, (mx + half).astype(np.int32), z,
+                             (mx - half).astype(np.int32), z, np.full(n, -10, np.int32), smp)
+
+
+@pytest.mark.parametrize("ns,repeat,ncdp,fold,spacing,apm,tau,na,nb,nc,amax,bmax,noise,early", [
+    (1500, 128, 5, 2, 5, 11, 1, 4, 9, 5, 3e-4, 1e-8, 1e-5, False),
+    (600, 1, 3, 17, 5, 21, 0, 4, 31, 7, 1e-5, 1e-8, 1e-5, False),
+    (300, 1, 5, 4, 5, 11, 0, 4, 5, 3, 1e-5, 4e-7, 1e-5, False),
+    (1000, 1, 2, 11, 12.5, 51, 0, 7, 31, 9, 1e-6, 1e-7, 1e-5, False),
+    (600, 1, 3, 6, 12.5, 13, 0, 4, 9, 12, 1e-5, 1.2e-6, 1e-6, True),
+    (600, 1, 5, 19, 12.5, 26, 1, 6, 31, 4, 1e-6, 2.8e-7, 1e-6, True),
+    (300, 40, 2, 1, 12.5, 51, 2, 3, 13, 12, 3e-4, 1.4e-8, 1e-5, True)])
+@pytest.mark.parametrize("form", ["plain", "f32"])
+def test_spikes_next_to_a_traveltime(form, ns, repeat, ncdp, fold, spacing, apm, tau, na, nb, nc, amax, bmax, noise, early):
+    if form != "plain":
+        tau = max(tau, 1)
+    prm = dict(a0=-amax, a1=amax, na=na, b0=-bmax, b1=bmax, nb=nb, c0=4e-7, c1=6e-7, nc=nc, aph=4000, apm=apm,
+               tau=tau * 0.004 * 1.0001, azimuth=0.0)
+    bad = 0
+    with semb.Plan(semb.params(semb.CRS, **_kw(form), **prm)) as p:
+        for seed in range(60):
+            arr = _spikes(np.random.default_rng(seed), ns, repeat, ncdp, fold, spacing, noise, early)
+            p.set_filter(semb.FILTER_ON)
+            p.upload(arr.view())
+            assert p.filter_tasks()[0] > 0
+            got = _results(p, form)
+            p.set_filter(semb.FILTER_OFF)
+            bad += sum(int((x != y).sum()) for x, y in zip(got, _results(p, form)))
+    assert bad == 0
+
+
 @pytest.mark.parametrize("form", ["f16", "bf16", "f32"])
 @pytest.mark.parametrize("seed", range(4))
 @pytest.mark.parametrize("tau", [1, 2])
