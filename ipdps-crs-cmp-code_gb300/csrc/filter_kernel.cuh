@@ -102,6 +102,7 @@ struct FilterParams {
   int2* fb_tasks;          // tasks whose lists overflowed
   int* fb_count;
   unsigned long long* fb_total;   // counts them over all launches of a run
+  float edge;              // within this of a sample boundary rounding may lie across it
   float kappa;             // multiple of the rms rounding effect (see above)
 };
 
@@ -421,8 +422,6 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
   const float q_lo = (float)(P.tau * P.tau), q_hi = (float)(P.ns - P.tau - 1) * (float)(P.ns - P.tau - 1);
   const float hdB = 0.5f * P.dB;
   const float sig = (float)P.ns * 5.9604645e-8f;   // t 2^-24 at the record's end
-  // within this of a sample boundary the direct kernel's rounding may lie across it
-  const float edge = 8.f * sig;
   float T = 0.f;
   // the warp's run: A, C and the centre's B; the real slots and their widest offset
   float ca = 0.f, cb = 0.f, cc = 0.f, rmax = 0.f;
@@ -504,7 +503,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
                           tg.cdp, t0);
           }
           ms.template add<QUAD>(a, x, k1, QUAD ? (k1 * k1) * ti : 0.f);
-          const float h = fmaf(k1, rmax, edge);
+          const float h = fmaf(k1, rmax, FP.edge);
           if (x + h >= 1.0f) um |= 1u << (e - 32 * b);
           if (x < h) dm |= 1u << (e - 32 * b);
         }
@@ -580,7 +579,7 @@ __global__ void __launch_bounds__(NT, 1) semb_filter_kernel(FilterParams FP) {
           ms.template add<true>(a, in ? x : 0.f, in ? k1 : 0.f, in ? (k1 * k1) * ti : 0.f);
         }
         if (in) {
-          const float hc = fmaf(k1, rmax, edge);
+          const float hc = fmaf(k1, rmax, FP.edge);
           const uint32_t up = x + hc >= 1.0f ? 1u << (e & 31) : 0u, dn = x < hc ? 1u << (e & 31) : 0u;
 #pragma unroll
           for (int b = 0; b < kMaxChunk / 32; ++b)

@@ -1410,6 +1410,7 @@ int enqueue_search(semb_plan* pl, const KernelCfg& cfg, const int2* tasks, int n
     F.fb_tasks = pl->d_fb_tasks;
     F.fb_count = pl->d_fb_count;
     F.fb_total = reinterpret_cast<unsigned long long*>(pl->d_fb_count + 6);
+    F.edge = 8.f * 5.9604645e-8f * (float)pl->ns;   // 8 t 2^-24 at the record's end
     F.kappa = form == FORM_PLAIN ? 16.f : 8.f;
     SEMB_TRY(launch_filter(form, pl->w, P.storage, f->shape, F, f->nwarps, std::min(ntasks, pl->sms), f->smem, st));
     RefineParams R{};
