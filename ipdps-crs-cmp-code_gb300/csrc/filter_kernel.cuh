@@ -7,7 +7,7 @@
 // best one in the plain form, the fourth best in the batched form, which keeps four).
 // The refine kernels (refine_kernel.cuh) then evaluate those few with the direct
 // kernels' own arithmetic, operation by operation, so the search's results are the
-// direct kernels'.
+// direct kernels' unless a candidate's rounding lies outside its bounds (see below).
 //
 // The items of one warp and lane are consecutive B values of one (A, C) pair: one run,
 // B_r = B_c + r dB about its centre slot.  On one trace their traveltimes differ by
@@ -60,20 +60,22 @@
 // per chunk.  The pipeline otherwise follows semb_pipe_kernel: a rotating planner warp,
 // mbarrier hand-offs, a work queue, the last warp of a task merging its lists.
 //
-// What bounds it: instruction issue.  On 16 CDPs of the 500 x 48 line with runs of 21 the
-// main loop (about 40 instructions per trace and run) issues on every cycle and takes 30%
-// of the time, the crossings (about 100 per noted trace of the busiest lane, on 56% of
-// cycles) 30%, the traces at the record's ends 10 to 15%, and the rest is the planner's and
-// the copies' latency, hidden only in part.  Long runs pay: 21 B values as one run of 22
+// What bounds it: the latency of a warp's own chains, at 12 warps of 168 registers per SM.
+// ncu on 16 CDPs of the 500 x 48 line: issue 59% of cycles, FMA pipe 34%, ALU 26%,
+// shared-memory loads 22%; a warp waits 1.3 cycles per instruction on fixed latencies, 0.65 on
+// instruction fetch, 0.6 on shared memory.  By section the main loop (about 40 instructions per
+// trace and run) takes 30% of the time, the crossings (about 100 per noted trace of the
+// busiest lane) 30%, the traces at the record's ends 10 to 15%, and the rest is the planner's
+// and the copies' latency, hidden only in part.  Long runs pay: 21 B values as one run of 22
 // slots at 384 threads took 29.5 ms where two runs of 12 slots at 512 threads took 36.2 (32
 // CDPs of the line), 31 as one of 32 slots at 256 threads 130 against 147 as two of 16.  The
 // second-order terms only where they count (moment_linear) gave 2%, the crossings above
 // and below the centre apart (half the slots each) 7%; two noted traces at a time was 10%
-// slower, and so was the main loop unrolled by four.
-// Measured on GB300, whole pass with the re-pick, before this kernel and now: 64 CDPs of
-// the line (21 x 21 x 21, FP16) 172.5 -> 53.6 ms; 128 CDPs with apertures of 50 to 2000
-// traces 449 -> 151 ms; 48 such CDPs with 31 x 31 x 31 candidates (BF16) 690 -> 189 ms;
-// plain form, 12 CDPs of the line 99.6 -> 9.4 ms.
+// slower, and so was the main loop unrolled by four.  Counting the steepest slopes costs 2 to 3%.
+// Measured on GB300, whole pass with the re-pick, with every candidate evaluated and now, in
+// turn on the same surveys: 64 CDPs of the line (21 x 21 x 21, FP16) 172.3 -> 55.4 ms; 128 CDPs
+// with apertures of 50 to 2000 traces 653 -> 206 ms; 48 such CDPs with 31 x 31 x 31 candidates
+// (BF16) 539 -> 178 ms; plain form, 12 CDPs of the line 99.6 -> 9.8 ms.
 #pragma once
 
 #include <type_traits>

@@ -80,7 +80,7 @@ static int plain_variant(int w, int ncand) {
 // staging and merges show on small folds: from 110 traces it pays with several passes a
 // chunk, from 150 with w = 1.  Measured, ring / two-barrier, folds of 30, 62 and 150: w = 5,
 // 160 candidates 0.83, 0.82, 0.81; 80 0.86, 0.81, 0.80; 256 1.11, 1.03, 0.95 (uneven folds of
-// 12 to 240 9.34 / 10.29 ms); 128 1.27, 1.12, 0.98; w = 3, 33 candidates 0.98, 0.88, 0.87; 64
+// 12 to 240 9.45 / 10.28 ms); 128 1.27, 1.12, 0.98; w = 3, 33 candidates 0.98, 0.88, 0.87; 64
 // 1.01, 0.99, 1.00; w = 1, 128 1.27, 1.06, 0.86.
 //
 // From w = 7 on the two-barrier kernel's entries of 16 bytes per window sample and its few
@@ -178,7 +178,7 @@ int launch_stt00(int w, int cdp0, int cdp1, const KParams& P, float a, float b, 
 // Items per warp: 32, so that one warp screens 32 consecutive items with one load each, but
 // fewer where that would leave the GPU's warps without work, as the near ties of a warp's
 // items run one after the other: 64 warps' worth of items per SM for CRS, most of whose items
-// are near ties (24 CDPs x 601 samples, w = 5: 3.2 ms at 32 per warp in FP64; 0.23 so, in
+// are near ties (24 CDPs x 601 samples, w = 5: 3.2 ms at 32 per warp in FP64; 0.26 so, in
 // pairs of FP32 numbers).  For CMP 1% are, and the screening of the others counts up to w = 5
 // (100 x 1000, w = 5: 44 us at 8 warps' worth, 54 at 32); a wider window's ties are the longer
 // ones (75 x 751, w = 11: 147 us at 8, 114 at 16, 109 at 32; 100 x 1000, w = 15: 183, 183, 136).
